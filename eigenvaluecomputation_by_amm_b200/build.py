@@ -36,7 +36,8 @@ def _sources():
 
 
 def _deps():
-    return _sources() + sorted(CSRC.glob("*.h")) + sorted(INCLUDE.glob("*.h"))
+    return (_sources() + sorted(CSRC.glob("*.h")) + sorted(CSRC.glob("*.cuh")) +
+            sorted(INCLUDE.glob("*.h")))
 
 
 def up_to_date(lib: Path = LIB) -> bool:

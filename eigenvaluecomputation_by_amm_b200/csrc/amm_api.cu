@@ -146,6 +146,11 @@ void layout(amm_ctx* ctx, Carver& cv) {
   b.spart = cv.take<float>(b.nsm);
   b.spart64 = cv.take<double>(b.nsm);
   b.rpart = cv.take<double>(4 * b.nsm);
+  // (amm_step.cu; one spare element each where that kernel is not used)
+  const int64_t pk = ctx->geom.packets ? amm::step_partial_packets(ctx->geom) : 0;
+  b.pk_part = cv.take<uint4>((size_t)b.nsm * pk);
+  b.pk_y = cv.take<uint4>(ctx->geom.packets ? amm::step_y_packets(ctx->geom) : 0);
+  b.epoch = cv.take<uint32_t>(1);
   b.colsum = cv.take<double2>(n);
   b.ticket = cv.take<uint32_t>(4);
   b.alpha2 = cv.take<double>(1);

@@ -108,6 +108,10 @@ struct Buffers {
   double* spart64;     // nsm  (Σ α_j² of each CTA, set-up)
   double2* colsum;     // n (Σa, Σa²) of each column from the set-up pass
   double* rpart;       // nsm x 4 (x·y, y·y, y·v*, z·dx) of each CTA
+  // packets of the step kernel (amm_step.cu): three floats and an epoch each
+  uint4* pk_part;      // nsm x (packets of a vector + 1): the CTAs' partial y and scalars
+  uint4* pk_y;         // packets of a vector: y; then the CTAs' shares of the Rayleigh sums
+  uint32_t* epoch;     // epoch before the next launch's first step
   uint32_t* ticket;    // [2]: grid-barrier arrivals of the step kernel and the set-up pass;
                        // [3]: the wait probe's barrier; [0], [1]: spare
   double* alpha2;      // ‖α‖²
@@ -143,7 +147,18 @@ struct PanelGeom {
   int stage_area;   // bytes reserved for the stages
   int smem_bytes;   // dynamic shared memory (set-up variant, the larger one)
   int wl_cap;       // work-list capacity per cluster
+  int packets;      // 1: the steps run in amm_step.cu's kernel (packet exchange), 0: in
+                    // amm_panel.cu's (clusters, or too few SMs)
 };
+
+// The step kernel of amm_step.cu: whether it covers a geometry, its dynamic shared memory, the
+// packets of one CTA's partial y (with its scalars) and of y (with the CTAs' shares), one
+// resident CTA per SM, and its launch.
+bool step_supported(const PanelGeom& g);
+int step_smem(const PanelGeom& g);
+int64_t step_partial_packets(const PanelGeom& g);
+int64_t step_y_packets(const PanelGeom& g);
+bool step_coresident(const PanelGeom& g);
 
 // cluster: requested CTAs per cluster (1, 2, 4 or 8; falls back to 1 where the shape or the
 // residency does not allow it).
@@ -205,6 +220,12 @@ cudaError_t launch_gather_alpha(const Buffers& b, int64_t count, cudaStream_t s)
 // [col0, col0 + n) of the c picks drawn from st_in (advanced into st_out, may alias).
 cudaError_t launch_shard_worklist(const Buffers& b, const double* cdf, int n_global, int col0,
                                   const uint32_t* st_in, uint32_t* st_out, int c, cudaStream_t s);
+
+// launch_iter_panel's form for geometries with packets = 1 (amm_step.cu).
+cudaError_t launch_step(const Buffers& b, const PanelGeom& g, const CallCfg& cc, int iter,
+                        int iter_end, cudaStream_t s);
+// The runtime accepts the cooperative attribute beside programmatic stream serialization.
+bool coop_with_pdl();
 
 // Count of this library's launches (for the bench's gpu_launches field).
 void count_launch(int k = 1);

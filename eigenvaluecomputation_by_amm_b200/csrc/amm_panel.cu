@@ -29,6 +29,7 @@
 
 #include "amm_device.cuh"
 #include "amm_internal.h"
+#include "amm_panel.cuh"
 
 namespace amm {
 
@@ -104,95 +105,6 @@ __host__ __device__ inline SmemLayout smem_layout(const PanelGeom& g, bool setup
   L.total = (o + 127) & ~127;
   return L;
 }
-
-// Packed FP32x2 arithmetic (Blackwell): two IEEE-rounded FMAs per instruction (the sm_100
-// builtin, so the compiler allocates the register pairs itself).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-// 16-byte vector -> E/2 float2 (exact for BF16: the 16 bits become the high half).
-__device__ __forceinline__ void unpack2(const uint4& v, float2 (&o)[2]) {
-  o[0] = make_float2(__uint_as_float(v.x), __uint_as_float(v.y));
-  o[1] = make_float2(__uint_as_float(v.z), __uint_as_float(v.w));
-}
-__device__ __forceinline__ void unpack2(const uint4& v, float2 (&o)[4]) {
-  o[0] = make_float2(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u));
-  o[1] = make_float2(__uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
-  o[2] = make_float2(__uint_as_float(v.z << 16), __uint_as_float(v.z & 0xffff0000u));
-  o[3] = make_float2(__uint_as_float(v.w << 16), __uint_as_float(v.w & 0xffff0000u));
-}
-
-// Branch-free body of one full group: the axpy of group g (stage `cur`, coefficients `coef`)
-// interleaved, slot by slot, with the partial dots of group g+1 (stage `nxt`) when NEXT.  Used
-// when every column of both groups is present and every vector slot of every thread is valid.
-template <typename Elem, int R, int GC, bool NEXT, int TC>
-__device__ __forceinline__ void fused_block(const unsigned char* cur, const unsigned char* nxt,
-                                            uint32_t col_bytes, int t, int T_rt,
-                                            const float (&coef)[GC],
-                                            const float2 (&dx)[R][8 / sizeof(Elem)],
-                                            float2 (&yacc)[R][8 / sizeof(Elem)], float (&dn)[GC]) {
-  constexpr int H = 8 / sizeof(Elem);
-  // with a compile-time thread count (TC > 0) every shared-memory load uses an immediate offset
-  const int T = TC > 0 ? TC : T_rt;
-  const int colv = TC > 0 ? R * TC : (int)(col_bytes >> 4);  // vectors per column
-  const uint4* c4 = reinterpret_cast<const uint4*>(cur) + t;
-  const uint4* n4 = reinterpret_cast<const uint4*>(nxt) + t;
-  float2 p[GC];
-#pragma unroll
-  for (int qq = 0; qq < GC; ++qq) p[qq] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    uint4 vc[GC], vn[GC];
-#pragma unroll
-    for (int qq = 0; qq < GC; ++qq) {
-      vc[qq] = c4[qq * colv + r * T];
-      if (NEXT) vn[qq] = n4[qq * colv + r * T];
-    }
-#pragma unroll
-    for (int qq = 0; qq < GC; ++qq) {
-      float2 ac[H];
-      unpack2(vc[qq], ac);
-      const float2 c2 = make_float2(coef[qq], coef[qq]);
-#pragma unroll
-      for (int h = 0; h < H; ++h) yacc[r][h] = fma2(c2, ac[h], yacc[r][h]);
-      if (NEXT) {
-        float2 an[H];
-        unpack2(vn[qq], an);
-#pragma unroll
-        for (int h = 0; h < H; ++h) p[qq] = fma2(an[h], dx[r][h], p[qq]);
-      }
-    }
-  }
-#pragma unroll
-  for (int qq = 0; qq < GC; ++qq) dn[qq] = p[qq].x + p[qq].y;
-}
-
-// Sum over the 16 warps of NC partial values per warp (element (w, c) at base[w * stride + c]),
-// computed identically by every warp: lane groups of L lanes own one value each and reduce by a
-// fixed xor tree (deterministic).
-template <typename V, int NC>
-__device__ __forceinline__ void warp_partials_sum(const V* base, int stride, int lane,
-                                                  V (&tot)[NC]) {
-  constexpr int L = (32 / NC) < 16 ? (32 / NC) : 16;  // lanes per value
-  constexpr int PER = 16 / L;                          // warp partials per lane
-  constexpr int CPR = 32 / L;                          // values per round
-  constexpr int ROUNDS = (NC + CPR - 1) / CPR;
-#pragma unroll
-  for (int rr = 0; rr < ROUNDS; ++rr) {
-    const int q = rr * CPR + lane / L;
-    const int w0 = lane % L;
-    V v = V(0);
-    if (q < NC) {
-#pragma unroll
-      for (int j = 0; j < PER; ++j) v += base[(w0 + j * L) * stride + q];
-    }
-#pragma unroll
-    for (int off = L / 2; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-#pragma unroll
-    for (int c = 0; c < CPR; ++c)
-      if (rr * CPR + c < NC) tot[rr * CPR + c] = __shfl_sync(0xffffffffu, v, c * L);
-  }
-}
-
 
 // Set-up variant of fused_block: the axpy uses coef = α_j; the next group's statistics are
 // per-vector FP32 partial sums of <= 8 values (BF16 squares are exact in FP32) folded into
@@ -1294,6 +1206,12 @@ bool panel_geometry(int m, int dtype, int c, int n, int nsm, int cluster, PanelG
   b.stage_bytes = stage;
   b.stage_area = ns * stage;
   b.wl_cap = probe.wl_cap;
+  // the step kernel's carve beside the set-up's: one stage fewer where that is what it takes
+  while (cluster == 1 && b.nstages > 3 && step_smem(b) > kSmemBudget) {
+    --b.nstages;
+    b.stage_area = b.nstages * stage;
+  }
+  b.packets = step_supported(b) ? 1 : 0;
   b.smem_bytes = smem_layout(b, true).total;
   *g = b;
   return b.smem_bytes <= kSmemBudget;
@@ -1313,7 +1231,7 @@ __global__ void coop_probe_kernel() {}
 
 static int g_coop_pdl[64] = {};  // per device: 0 unknown, 1 accepted, 2 refused
 
-static bool coop_with_pdl() {
+bool coop_with_pdl() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
   if (g_coop_pdl[dev] == 0) {
@@ -1378,6 +1296,7 @@ bool panel_coresident(PanelGeom* g, int nsm) {
       fit = std::min(fit, nc);
     }
   }
+  if (g->packets && !step_coresident(*g)) g->packets = 0;
   if (g->cluster > 1) {
     if (fit * g->cluster < nsm / 2) return false;  // the work lists are sized for >= nsm/2 CTAs
     g->nclusters = fit;
@@ -1436,6 +1355,7 @@ cudaError_t launch_setup_panel(const Buffers& b, const PanelGeom& g, cudaStream_
 
 cudaError_t launch_iter_panel(const Buffers& b, const PanelGeom& g, const CallCfg& cc, int iter,
                               int iter_end, cudaStream_t s) {
+  if (g.packets) return launch_step(b, g, cc, iter, iter_end, s);
   PanelArgs a{};
   a.b = b;
   a.g = g;

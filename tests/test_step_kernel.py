@@ -1,0 +1,61 @@
+"""The persistent step kernel's packet exchange and its two product forms on the B200, against the
+oracle: shapes at the edges of the packet ownership (fewer packets than CTAs, a last packet of one
+or two values, rows that do not fill the block), slices that just fit the shared-memory ring and
+slices that do not, several launches per call, and an eigenvector for the error trace.
+
+Tolerances: λ within helpers.RTOL_LAMBDA_F32, the final vector within 1e-4 (FP32 dots and partial
+sums against the FP64-accumulating oracle), states and step kinds exactly.
+"""
+import numpy as np
+import pytest
+import torch
+
+import amm_oracle as O
+from helpers import RTOL_LAMBDA_F32, rel, scaled_gaussian, states, vec_rel
+
+pytestmark = pytest.mark.gpu
+
+# (m, n, c, dtype): 4 values per thread and fewer packets than CTAs; one more row group than a
+# block of 32 threads; 8 rows per thread with idle threads (3000 BF16 rows as 375 vectors of 384);
+# 16 and 32 rows per thread, full and not; a resident slice (n / 148 columns within the ring) and a
+# streamed one for the same m
+SHAPES = [(4, 400, 20, "f32"), (132, 300, 40, "f32"), (1024, 700, 90, "f32"),
+          (1024, 9000, 500, "f32"), (2052, 1500, 150, "f32"), (8192, 900, 130, "f32"),
+          (8196, 600, 77, "f32"), (16380, 700, 150, "f32"), (8, 300, 33, "bf16"),
+          (3000, 2111, 301, "bf16"), (8200, 801, 99, "bf16"), (16384, 1300, 200, "bf16")]
+
+
+@pytest.mark.parametrize("method,kw", [("exact", {}), ("previous", dict(vr_period=5)),
+                                       ("proposed", dict(vr_period=4))])
+@pytest.mark.parametrize("m,n,c,dtype", SHAPES)
+def test_step_kernel_shapes(m, n, c, dtype, method, kw):
+    from eigenvaluecomputation_by_amm_b200 import AMMContext, column_major
+    step = 18                                      # two launches for the sampled methods
+    A = scaled_gaussian(m, n, seed=m + n, shift=0.05)
+    tA = torch.from_numpy(A).cuda()
+    if dtype == "bf16":
+        tA = tA.to(torch.bfloat16)
+        A = tA.float().cpu().numpy()
+    ctx = AMMContext(m, n, c=c, step=step, dtype=dtype, **kw)
+    ctx.set_matrix(column_major(tA))
+    st = states(c, m + c)
+    ctx.set_rng_state(torch.from_numpy(st.view(np.int32)).cuda())
+    x0 = np.random.default_rng(m + 5).standard_normal(m).astype(np.float32)
+    vstar = np.random.default_rng(m + 6).standard_normal(m)
+    vstar /= np.linalg.norm(vstar)
+    ctx.set_eigenvector(torch.from_numpy(vstar))
+    ctx.power_method(method, torch.from_numpy(x0).cuda())
+    tr = ctx.trace()
+    ref = O.power_method(A, x0, method=method, step=step, c=c, states=st, vstar=vstar, **kw)
+    assert tr["kinds"] == ref.modes
+    assert np.all(rel(tr["eigs"], ref.eigs) < RTOL_LAMBDA_F32), rel(tr["eigs"], ref.eigs)
+    assert np.all(np.abs(tr["errs"] - ref.errs) < 1e-4)
+    if method != "exact":
+        assert np.array_equal(ctx.get_rng_state(c).cpu().numpy().view(np.uint32), ref.states[:c])
+    x, _ = ctx.vectors()
+    assert vec_rel(x.cpu().numpy(), ref.x) < 1e-4
+    # the same call again: bitwise the same (fixed orders throughout, epochs that move on)
+    ctx.set_rng_state(torch.from_numpy(st.view(np.int32)).cuda())
+    ctx.power_method(method, torch.from_numpy(x0).cuda())
+    assert np.array_equal(ctx.trace()["eigs"], tr["eigs"])
+    ctx.close()
