@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "amm.h"
+#include "amm_batch.h"
 #include "amm_device.cuh"
 #include "amm_internal.h"
 
@@ -49,16 +50,6 @@ constexpr int kJacobiSweeps = 16;
 constexpr int kMaxCols = 8192;   // AMM mode: the CDF lives in shared memory
 constexpr int kVrSlot = 3;       // VR scratch per CTA: X_memo, Y_memo, saved X
 constexpr int kMaxPicks = 1024;  // AMM mode: c <= n / 8
-
-struct Mat {
-  const float* A;  // column-major, ld % 4 == 0, 16-byte aligned
-  int64_t ld;
-  int32_t m, n;
-  int64_t out_off;  // first row of this matrix's vector in the output
-  int64_t st_off;   // AMM mode: first of this matrix's c xorshift states
-  int32_t c;        // AMM mode: samples per product (0: exact)
-  int32_t pad;
-};
 
 struct Args {
   const Mat* mats;
@@ -289,6 +280,7 @@ struct Smem {
   static constexpr int region = TC ? align1024(xs + xs_bytes) : align16(xs + xs_bytes);
   static constexpr int yred = region;                                    // float [4*kThreads][K]
   static constexpr int hist = align16(yred + 4 * kThreads * K * 4);      // uint32 [kMaxCols]
+  static constexpr int xrow = hist;  // tensor-core kernel, a matrix multiplied as C·X: X as [row][v]
   static constexpr int region_bytes =
       TC ? cmax(2 * kTcStageFloats * 4, 4 * kThreads * K * 4)
          : cmax(hist + kMaxCols * 4 - region, kRingBytes);
@@ -301,6 +293,7 @@ struct Smem {
   static constexpr int total_amm = align16(svr + K * K * 4);
   static_assert(gpart % 8 == 0 && cs % 8 == 0 && xs % 16 == 0 && region % 16 == 0,
                 "shared-memory alignment");
+  static_assert(!TC || xrow + kMaxRows * K * 4 <= region + region_bytes, "X by row fits the region");
   static_assert(!TC || total <= 227 * 1024, "the tensor-core layout exceeds a CTA's shared memory");
 };
 
@@ -683,6 +676,103 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
   }
 }
 
+// Y = C·X over this team's share of C's columns (C = A·Aᵀ, ldc x ldc, zeros past m), this thread's
+// rows r0 .. r0 + 3, for an even number of vectors: per column one 16-byte load of C (coalesced
+// over the team, four columns ahead in registers) against X's row (broadcast loads: `xrow` [row][v],
+// or without it the interleaved pairs of Xs), in packed FP32 FMAs.  Bounded by the FMAs and by an
+// SM's share of the L2 (16 packed FMAs per 16 bytes).  The sums are taken in runs of 16 columns, added
+// up in this thread's slot of shared memory (`slots`, [value / 4][thread]): one FP32 chain over a
+// team's whole share made the rounding of Y the largest error of λ where the eigenvector sits on
+// few rows (300 x 700 with lognormal row scales: rms 1.6e-7 -> 1.2e-7).  Out of line so that its
+// registers do not compete with the other product loops'.
+template <int K>
+__device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, const float* xrow,
+                                        const float* Xs, float4* slots, int r0, int g0, int gstep,
+                                        float (&Y)[4][K]) {
+  constexpr int KP = K / 2;
+  float2 run[4][KP];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int p = 0; p < KP; ++p) run[e][p] = make_float2(0.f, 0.f);
+  const int ng = ldc >> 2;  // groups of 4 columns
+  const float* base = C + r0;
+  float4 c[4], cn[4];
+  auto load = [&](int g, float4 (&o)[4]) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      o[j] = __ldg(reinterpret_cast<const float4*>(base + (int64_t)(4 * g + j) * ldc));
+  };
+  bool some = false;  // the slot holds earlier runs
+  float4* slot = slots + threadIdx.x;
+  auto add_slot = [&]() {  // run += slot
+    if (some)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int p = 0; p < KP; p += 2) {
+          const float4 v = slot[(e * KP + p) / 2 * kThreads];
+          run[e][p] = __fadd2_rn(run[e][p], make_float2(v.x, v.y));
+          run[e][p + 1] = __fadd2_rn(run[e][p + 1], make_float2(v.z, v.w));
+        }
+  };
+  if (r0 < ldc && g0 < ng) {
+    load(g0, cn);
+    int left = 4;  // groups of the run
+#pragma unroll 1
+    for (int g = g0; g < ng; g += gstep) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c[j] = cn[j];
+      if (g + gstep < ng) load(g + gstep, cn);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float2 x[KP];
+        const int k = 4 * g + j;
+        if (xrow) {
+#pragma unroll
+          for (int p = 0; p < KP; p += 2) {
+            const float4 v = *reinterpret_cast<const float4*>(xrow + k * K + 2 * p);
+            x[p] = make_float2(v.x, v.y);
+            x[p + 1] = make_float2(v.z, v.w);
+          }
+        } else {
+#pragma unroll
+          for (int p = 0; p < KP; ++p)
+            x[p] = *reinterpret_cast<const float2*>(Xs + p * 2 * kMaxRows + 2 * k);
+        }
+        const float ce[4] = {c[j].x, c[j].y, c[j].z, c[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 d = make_float2(ce[e], ce[e]);
+#pragma unroll
+          for (int p = 0; p < KP; ++p) run[e][p] = __ffma2_rn(d, x[p], run[e][p]);
+        }
+      }
+      if (--left == 0 && g + gstep < ng) {
+        add_slot();
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int p = 0; p < KP; p += 2) {
+            slot[(e * KP + p) / 2 * kThreads] =
+                make_float4(run[e][p].x, run[e][p].y, run[e][p + 1].x, run[e][p + 1].y);
+            run[e][p] = run[e][p + 1] = make_float2(0.f, 0.f);
+          }
+        some = true;
+        left = 4;
+      }
+    }
+    add_slot();
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+#pragma unroll
+    for (int p = 0; p < KP; ++p) {
+      Y[e][2 * p] = run[e][p].x;
+      Y[e][2 * p + 1] = run[e][p].y;
+    }
+}
+
 template <int K, int GC, bool TC = false>
 __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constant__ Args a) {
   constexpr int NV = K * GC;
@@ -964,6 +1054,11 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
           }
 #pragma unroll
           for (int e = 0; e < 4; ++e) Xs[xs_idx<K, TC>(j, r0 + e)] = xj[e];
+          if (TC && M.C) {  // X by row for the product with C (in the idle tile region)
+            float* xr = reinterpret_cast<float*>(smem + SL::xrow);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) xr[(r0 + e) * K + j] = xj[e];
+          }
         }
       }
       __syncthreads();
@@ -1041,7 +1136,13 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // ---- Y = C·X (or its AMM estimate): the fused pass over the columns (team-local) ----
       const bool rows = r0 < m;
       int buf = 0;
-      if constexpr (TC) {
+      const bool by_c = K % 2 == 0 && M.C != nullptr && !wamm;  // an exact product as C·X
+      if (by_c) {
+        if constexpr (K % 2 == 0)
+          cx_product<K>(M.C, M.ldc, TC ? reinterpret_cast<const float*>(smem + SL::xrow) : nullptr,
+                        Xs, reinterpret_cast<float4*>(yred), r0, gteam, NTG, Y);
+        __syncthreads();  // the slots lie where Y is copied next
+      } else if constexpr (TC) {
         // ---- tensor-core pass (exact mode, 8 vectors).  Warp wi of a team owns the team's
         // rows [128·wi, 128·wi + 128); per group of 8 columns its lane 0 copies those rows into
         // the warp's own 4 KB tile (two stages) with four TMA boxes of 32 rows x 8 columns
@@ -1314,7 +1415,7 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       cp_async_wait_all();  // only empty groups can still be open here
       }
       // ---- sum the team partials of Y (fixed order), every team receives the total ----
-      if (!TC && NT > 1) {
+      if ((!TC || by_c) && NT > 1) {
         __syncthreads();
         if (rows) {
 #pragma unroll
@@ -1549,6 +1650,11 @@ struct amm_batch {
   int64_t total_cols = 0;
   int64_t n_states = 0;
   bool amm = false;
+  // matrices multiplied as C·X: the tiles of their C = A·Aᵀ (longest first) and C's memory
+  float* c_mem = nullptr;
+  amm::batch::GramTile* d_tiles = nullptr;
+  int ntiles = 0;
+  std::vector<double> cost;  // estimated clocks of a run per matrix, for the order and the plan
   // device memory (one allocation)
   void* mem = nullptr;
   Mat* d_mats = nullptr;
@@ -1651,11 +1757,13 @@ int persistent_grid(amm_batch* b, int variant, int cl) {
 
 // Start of a run: both work-list counters zeroed and, in AMM mode, the seeded states restored
 // (every run draws the same picks).
-int run_prologue(amm_batch* b, cudaStream_t s) {
-  BATCH_CUDA(cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(uint32_t), s));
+int run_prologue(amm_batch* b, cudaStream_t s, bool gram = true) {
+  BATCH_CUDA(cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(uint32_t), s));
   if (b->amm)
     BATCH_CUDA(cudaMemcpyAsync(b->d_states, b->d_states0, sizeof(uint32_t) * b->n_states,
                                cudaMemcpyDeviceToDevice, s));
+  if (gram && b->ntiles > 0)
+    BATCH_CUDA(amm::batch::launch_gram(b->d_mats, b->d_tiles, b->ntiles, b->d_queue + 2, b->nsm, s));
   return AMM_OK;
 }
 
@@ -1716,8 +1824,9 @@ int launch_kernel(amm_batch* b, int variant, int cl, int grid, double* d_lam, fl
 
 // A run as one launch over the order list (or a slice of it).
 int launch(amm_batch* b, int variant, int cl, int grid, double* d_lam, float* d_vec,
-           int32_t* d_iters, int max_iter, const int32_t* order, int count, cudaStream_t s) {
-  const int rc = run_prologue(b, s);
+           int32_t* d_iters, int max_iter, const int32_t* order, int count, cudaStream_t s,
+           bool gram = true) {
+  const int rc = run_prologue(b, s, gram);
   if (rc) return rc;
   return launch_kernel(b, variant, cl, grid, d_lam, d_vec, d_iters, max_iter, order, count,
                        nullptr, 0, false, s);
@@ -1759,11 +1868,11 @@ void plan_wide(amm_batch* b) {
   if (!amm::pdl_enabled() || b->cfg.wide < 0 || b->count < 2) return;
   if (b->cfg.cluster > 0 && b->cfg.wide == 0) return;
   double total = 0.0;
-  for (const Mat& x : b->mats) total += (double)x.m * (double)x.n;
+  for (const double c : b->cost) total += c;
   // work per SM of an even split, with a margin: the per-CTA rate falls with the row count,
   // so the heaviest matrices are also the slowest per element
   const double share = 0.75 * total / (double)b->nsm;
-  auto work = [&](int k) { const Mat& x = b->mats[b->order[k]]; return (double)x.m * x.n; };
+  auto work = [&](int k) { return b->cost[b->order[k]]; };
   int nwide = 0;
   while (nwide < b->count && work(nwide) > (double)b->cluster * share) ++nwide;
   if (nwide == 0) return;
@@ -1805,6 +1914,10 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   for (int v = 0; v < n_var; ++v) {
     if (amm::batch::kVariants[v].K != b->cfg.nvec) continue;
     if (amm::batch::kVariants[v].tc && (b->amm || !b->d_tmaps)) continue;  // exact-only, maps
+    // with products as C·X the tile shape matters to the other matrices alone: only the best
+    // exact one is tried
+    if (b->ntiles > 0 && !b->amm && b->d_tmaps && b->cfg.nvec == 8 && !amm::batch::kVariants[v].tc)
+      continue;
     if (b->cfg.tile_gc > 0 && amm::batch::kVariants[v].GC != b->cfg.tile_gc) continue;
     for (int cl : amm::batch::kClusterSizes) {
       if (b->cfg.cluster > 0 && cl != b->cfg.cluster) continue;
@@ -1941,6 +2054,73 @@ static bool encode_tensor_maps(const std::vector<Mat>& ms, std::vector<CUtensorM
   return true;
 }
 
+// Exact products of a run (a tolerance may stop it earlier: 16 are counted then).
+static double exact_products(const amm_batch_config& cfg) {
+  const int64_t it = cfg.max_iter;
+  if (cfg.c_divisor > 0) {
+    if (cfg.vr_period <= 0) return 0.0;
+    return (double)(it / cfg.vr_period + (it % cfg.vr_period != 0 ? 1 : 0));
+  }
+  return (double)(cfg.tol > 0.0 ? std::min<int64_t>(it, 16) : it);
+}
+
+// Estimated clocks of one SM for a run's products of a matrix through A: 11 bytes of A a clock on the
+// tensor-core product, 8.5 on the CUDA-core one (C4, measured).
+static double direct_clocks(const Mat& x, const amm_batch_config& cfg) {
+  const double rate = cfg.nvec == 8 && cfg.c_divisor == 0 ? 11.0 : 8.5;
+  const double p = cfg.c_divisor > 0
+                       ? exact_products(cfg) + (double)cfg.max_iter / (double)cfg.c_divisor
+                       : exact_products(cfg);
+  return p * 4.0 * (double)x.m * (double)x.n / rate;
+}
+
+// Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which forming C
+// (2500 clocks per 128 x 128 tile and 64 columns) and the products with it (m·m·nvec FMAs at 128 a
+// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only with the tile shape
+// left to the library (a fixed one asks for its product) and an even block.  Returns C's floats
+// in all; `cost`: estimated clocks per matrix.
+static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg,
+                         std::vector<double>& cost) {
+  const double p = exact_products(cfg);
+  int64_t floats = 0;
+  cost.resize(ms.size());
+  for (size_t i = 0; i < ms.size(); ++i) {
+    Mat& x = ms[i];
+    x.C = nullptr;
+    x.ldc = (x.m + 3) / 4 * 4;
+    const double direct = p * 4.0 * (double)x.m * (double)x.n /
+                          (cfg.nvec == 8 && cfg.c_divisor == 0 ? 11.0 : 8.5);
+    const double t = (double)((x.m + 127) / 128), chunks = (double)((x.n + 63) / 64);
+    const double form = t * (t + 1) / 2 * chunks * 2500.0;
+    const double by_c = p * (double)x.m * (double)x.m * (double)cfg.nvec / 96.0;
+    cost[i] = direct_clocks(x, cfg);
+    if (cfg.tile_gc == 0 && cfg.nvec % 2 == 0 && form + by_c < 0.8 * direct) {
+      x.C = reinterpret_cast<float*>(1);  // placed by place_gram
+      floats += (int64_t)x.ldc * x.ldc;
+      cost[i] += by_c - direct;  // (C is formed by a launch of its own)
+    }
+  }
+  return floats;
+}
+
+// C of the planned matrices in `mem`, and their tiles, longest first.
+static void place_gram(std::vector<Mat>& ms, float* mem, std::vector<amm::batch::GramTile>& tiles) {
+  int64_t off = 0;
+  for (size_t i = 0; i < ms.size(); ++i) {
+    Mat& x = ms[i];
+    if (!x.C) continue;
+    x.C = mem + off;
+    off += (int64_t)x.ldc * x.ldc;
+    const int t = (x.m + 127) / 128;
+    for (int ti = 0; ti < t; ++ti)
+      for (int tj = 0; tj <= ti / 2; ++tj) tiles.push_back({(int32_t)i, ti, tj, 0});
+  }
+  std::stable_sort(tiles.begin(), tiles.end(),
+                   [&](const amm::batch::GramTile& a, const amm::batch::GramTile& c) {
+                     return ms[a.mat].n > ms[c.mat].n;
+                   });
+}
+
 int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t count,
                      const amm_batch_config* cfg, int device) {
   if (!out || !mats || !cfg || count < 1 || count > (1 << 20)) return AMM_ERR_INVALID_ARGUMENT;
@@ -1979,10 +2159,25 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
     off += x.m;
     cols += x.n;
   }
+  std::vector<double> cost;
+  const int64_t c_floats = plan_gram(ms, *cfg, cost);
   amm_batch* b = new amm_batch();
   b->device = device;
   b->cfg = *cfg;
   b->count = count;
+  Guard g(device);
+  // C of the matrices multiplied as C·X (an allocation of its own: without room for it every
+  // product reads A)
+  if (c_floats > 0 && cudaMalloc(&b->c_mem, sizeof(float) * (size_t)c_floats) != cudaSuccess) {
+    cudaGetLastError();
+    b->c_mem = nullptr;
+    for (Mat& x : ms) x.C = nullptr;
+    for (int64_t i = 0; i < count; ++i) cost[i] = direct_clocks(ms[i], *cfg);
+  }
+  std::vector<amm::batch::GramTile> tiles;
+  if (b->c_mem) place_gram(ms, b->c_mem, tiles);
+  b->ntiles = (int)tiles.size();
+  b->cost = cost;
   b->mats = ms;
   b->vec_len = off;
   b->total_cols = cols;
@@ -1990,11 +2185,9 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   b->amm = amm_mode;
   b->order.resize((size_t)count);
   for (int64_t i = 0; i < count; ++i) b->order[i] = (int32_t)i;
-  // largest first (work m·n), ties by index: the queue then balances like LPT scheduling
-  std::stable_sort(b->order.begin(), b->order.end(), [&](int32_t x, int32_t y) {
-    return (int64_t)ms[x].m * ms[x].n > (int64_t)ms[y].m * ms[y].n;
-  });
-  Guard g(device);
+  // largest first (estimated clocks), ties by index: the queue then balances like LPT scheduling
+  std::stable_sort(b->order.begin(), b->order.end(),
+                   [&](int32_t x, int32_t y) { return cost[x] > cost[y]; });
   cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, device);
   size_t bytes = 0;
   auto carve = [&](size_t n, size_t align) {
@@ -2018,9 +2211,11 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   const size_t o_vr = with_vr ? carve(sizeof(float) * vr_floats * b->nsm, 256) : 0;
   // tensor maps (64-byte aligned each) when the tensor-core kernel can run: exact, 8 vectors
   const bool with_tmaps = !amm_mode && cfg->nvec == 8 && encode_tensor_maps(ms, b->h_tmaps);
+  const size_t o_tiles = carve(sizeof(amm::batch::GramTile) * (tiles.empty() ? 1 : tiles.size()), 256);
   const size_t o_tmaps = with_tmaps ? carve(sizeof(CUtensorMap) * count, 256) : 0;
   cudaError_t e = cudaMalloc(&b->mem, bytes);
   if (e != cudaSuccess) {
+    if (b->c_mem) cudaFree(b->c_mem);
     delete b;
     return e == cudaErrorMemoryAllocation ? AMM_ERR_OUT_OF_MEMORY : fail(e, "cudaMalloc");
   }
@@ -2035,6 +2230,7 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   b->d_states = reinterpret_cast<uint32_t*>(base + o_st);
   b->d_vr = with_vr ? reinterpret_cast<float*>(base + o_vr) : nullptr;
   b->d_tmaps = with_tmaps ? reinterpret_cast<CUtensorMap*>(base + o_tmaps) : nullptr;
+  b->d_tiles = reinterpret_cast<amm::batch::GramTile*>(base + o_tiles);
   std::vector<int64_t> cs((size_t)count + 1, 0);
   for (int64_t i = 0; i < count; ++i) cs[i + 1] = cs[i] + ms[i].n;
   e = cudaMemcpy(b->d_mats, ms.data(), sizeof(Mat) * count, cudaMemcpyHostToDevice);
@@ -2042,6 +2238,9 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
     e = cudaMemcpy(b->d_order, b->order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(b->d_col_start, cs.data(), sizeof(int64_t) * (count + 1),
+                   cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && !tiles.empty())
+    e = cudaMemcpy(b->d_tiles, tiles.data(), sizeof(tiles[0]) * tiles.size(),
                    cudaMemcpyHostToDevice);
   if (e == cudaSuccess && with_tmaps)
     e = cudaMemcpy(b->d_tmaps, b->h_tmaps.data(), sizeof(CUtensorMap) * count,
@@ -2063,6 +2262,7 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   }
   if (e != cudaSuccess) {
     cudaFree(b->mem);
+    if (b->c_mem) cudaFree(b->c_mem);
     delete b;
     return fail(e, "cudaMemcpy(batch descriptors)");
   }
@@ -2077,6 +2277,7 @@ int amm_batch_destroy(amm_batch* b) {
   if (b->graph) cudaGraphDestroy(b->graph);
   if (b->cap) cudaStreamDestroy(b->cap);
   if (b->mem) cudaFree(b->mem);
+  if (b->c_mem) cudaFree(b->c_mem);
   delete b;
   return AMM_OK;
 }
@@ -2126,7 +2327,7 @@ int amm_batch_run(amm_batch* b, double* d_lambda, float* d_vectors, int32_t* d_i
     b->g_iters = d_iters;
   }
   BATCH_CUDA(cudaGraphLaunch(b->gexec, s));
-  amm::count_launch(b->wide_count > 0 ? 2 : 1);
+  amm::count_launch((b->wide_count > 0 ? 2 : 1) + (b->ntiles > 0 ? 1 : 0));
   return AMM_OK;
 }
 
@@ -2141,7 +2342,7 @@ int amm_batch_run_each(amm_batch* b, double* d_lambda, float* d_vectors, int32_t
   // the order array
   for (int64_t i = 0; i < b->count; ++i) {
     rc = launch(b, b->variant, b->cluster, b->cluster, d_lambda, d_vectors, d_iters,
-                (int)b->cfg.max_iter, b->d_order + i, 1, s);
+                (int)b->cfg.max_iter, b->d_order + i, 1, s, i == 0);  // (C of every matrix once)
     if (rc) return rc;
   }
   return AMM_OK;
