@@ -73,7 +73,7 @@ struct Args {
   int32_t vr_base;   // first slot of this launch's CTAs in vr_mem (the second launch of a run
                      // is offset past the first one's CTAs)
   float* vr_mem;     // per CTA slot: X_memo, Y_memo, then X saved while a sampled product
-                     // multiplies D in its place; kMaxRows x K floats each ([row][v])
+                     // multiplies D in its place; kMaxRows x K floats each (see memo_load)
   // optional record for parity checks (null: none): each matrix's FP32 CDF at col_start[mi]
   // and the raw picks of its AMM product p < rec_products at st_off·rec_products + p·c + k
   float* rec_cdf;
@@ -113,6 +113,48 @@ __device__ __forceinline__ int xs_idx(int v, int row) {
     return v * kMaxRows + row;
 }
 
+// Shared-memory layout of Y (and of X by row): a thread's 4 rows x K vectors are K float4s (value
+// e·K + v of row 4·slot + e in float4 (e·K + v) / 4), permuted by the slot so that 8 neighbouring
+// threads' accesses of the same float4 fall on different banks (unpermuted, 128 bytes apart, they
+// all fall on one).
+template <int K>
+__device__ __forceinline__ int yq(int slot, int i) {
+  if constexpr (K == 8)
+    return slot * 8 + (i ^ (slot & 7));
+  else if constexpr (K == 4)
+    return slot * 4 + (i ^ ((slot >> 1) & 3));
+  else
+    return slot * K + i;
+}
+// the same for one value (a float offset)
+template <int K>
+__device__ __forceinline__ int yat(int row, int v) {
+  const int k = (row & 3) * K + v;
+  return 4 * yq<K>(row >> 2, k >> 2) + (k & 3);
+}
+template <int K>
+__device__ __forceinline__ void y_store(float* dst, int slot, const float (&Y)[4][K]) {
+#pragma unroll
+  for (int i = 0; i < K; ++i)
+    reinterpret_cast<float4*>(dst)[yq<K>(slot, i)] =
+        make_float4(Y[4 * i / K][4 * i % K], Y[(4 * i + 1) / K][(4 * i + 1) % K],
+                    Y[(4 * i + 2) / K][(4 * i + 2) % K], Y[(4 * i + 3) / K][(4 * i + 3) % K]);
+}
+// Y = src (ADD: Y += src)
+template <int K, bool ADD>
+__device__ __forceinline__ void y_load(const float* src, int slot, float (&Y)[4][K]) {
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const float4 v = reinterpret_cast<const float4*>(src)[yq<K>(slot, i)];
+    const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float& y = Y[(4 * i + c) / K][(4 * i + c) % K];
+      y = ADD ? y + w[c] : w[c];
+    }
+  }
+}
+
 // Start block: a counter-based hash of (seed, matrix, row, vector) -> uniform [-1, 1).
 __device__ __forceinline__ float start_value(uint64_t seed, int mi, int row, int v) {
   uint64_t z = seed ^ (0x9E3779B97F4A7C15ull * (uint64_t)(mi + 1)) ^
@@ -138,101 +180,124 @@ __device__ __forceinline__ void rr_pair(int K, int r, int s, int* p, int* q) {
   *q = a < b ? b : a;
 }
 
+// 1/sqrt(x) to FP64 rounding for x in FP32's normal range: two of Newton's steps from the FP32
+// reciprocal square root, without a branch (so that two of them interleave)
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  double y = (double)rsqrtf((float)x);
+  const double hx = 0.5 * x;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) y *= fma(-(hx * y), y, 1.5);
+  return y;
+}
+
+// The rotation (c, s) that annihilates h_pq: d = h_qq − h_pp, b = 2·h_pq, cos 2θ = |d|/h, sin 2θ =
+// sign(d)·b/h, h = sqrt(d² + b²); entries scaled to at most about 1 (below 1e-18 of that there is
+// nothing to rotate).
+__device__ __forceinline__ void jacobi_angle(double hpp, double hqq, double hpq, double* c,
+                                             double* s) {
+  const double d = hqq - hpp, b = hpq + hpq;
+  const double h2 = fma(d, d, b * b);
+  const double rh = rsqrt_newton(h2);
+  const double c2 = fma(0.5 * fabs(d), rh, 0.5);  // cos²θ, in [1/2, 1]
+  const double rc = rsqrt_newton(c2);
+  const bool rot = hpq != 0.0 && h2 > 1e-36;
+  *c = rot ? c2 * rc : 1.0;
+  *s = rot ? copysign(0.5, d) * (b * rh) * rc : 0.0;
+}
+
 // Cyclic Jacobi on the symmetric K x K matrix H (FP64, shared memory) by one warp; V receives
-// the eigenvectors (columns), H the eigenvalues on its diagonal.  Rotations of one round act on
-// disjoint index pairs, so a round is applied in parallel: lane = pair slot * K + index.
+// the eigenvectors (columns), H the eigenvalues on its diagonal.  The rotations of a round act on
+// disjoint index pairs, so a round is applied at once: lane (a, b) holds the 2 x 2 block of H in
+// rows of pair a and columns of pair b and rotates it from both sides; the lanes after those hold
+// one row of V in two pairs each.  Every lane forms the two angles it needs itself, from entries
+// loaded beside its block: a round is one shared-memory read, two interleaved angles, one write and
+// two warp barriers.
 template <int K>
-__device__ void jacobi_warp(double* H, double* V, double* cs, int lane) {
+__device__ void jacobi_warp(double* H, double* V, int lane) {
+  __builtin_assume(__isShared(H));
+  __builtin_assume(__isShared(V));
   for (int i = lane; i < K * K; i += 32) V[i] = (i / K == i % K) ? 1.0 : 0.0;
   __syncwarp();
-  if constexpr (K == 1) return;
-  for (int sweep = 0; sweep < kJacobiSweeps; ++sweep) {
-    double off = 0.0, dia = 0.0;
-    for (int i = lane; i < K * K; i += 32) {
-      const double h = H[i];
-      if (i / K == i % K)
-        dia += h * h;
-      else
-        off += h * h;
-    }
-    off = warp_sum(off);
-    dia = warp_sum(dia);
-    // off-diagonal entries below ~1e-13 of the matrix: the eigenvalue error left is their
-    // square over the gap (the FP64 rounding floor of `off` is ~K²·eps²·dia, so a tighter test
-    // would never be met and run every sweep); also stops on NaN
-    if (!(off > 1e-26 * dia)) break;
-    for (int r = 0; r < K - 1; ++r) {
-      if (lane < K / 2) {
-        int p, q;
-        rr_pair(K, r, lane, &p, &q);
-        const double hpq = H[p * K + q];
-        double c = 1.0, s = 0.0;
-        if (hpq != 0.0) {
-          // t = tan θ = sign(d)·b / (|d| + sqrt(d² + b²)), d = h_qq − h_pp, b = 2·h_pq (the
-          // annihilating angle), to FP32 accuracy from d and b scaled by an exact power of two
-          // (max(|d|, |b|) in [1, 2)); (c, s) = (1, t)/sqrt(1 + t²) in FP32, then two Newton
-          // steps x <- x·(3 − (c² + s²))/2 in FP64 make the rotation orthogonal to FP64
-          // rounding.  An angle off by FP32 rounding leaves h_pq at ~1e-7 of its size instead of
-          // 0, which the next sweep removes; the eigenvalues depend only on the orthogonality.
-          const double dd = H[q * K + q] - H[p * K + p], bb = 2.0 * hpq;
-          const double mx = fmax(fabs(dd), fabs(bb));
-          const int ex = (int)((__double_as_longlong(mx) >> 52) & 0x7ff);
-          const double sc = __longlong_as_double((long long)(2046 - min(ex, 2045)) << 52);
-          const float df = (float)(dd * sc), bf = (float)(bb * sc);
-          const float tf = copysignf(1.f, df) *
-                           __fdividef(bf, fabsf(df) + sqrtf(fmaf(df, df, bf * bf)));
-          const float cf = rsqrtf(fmaf(tf, tf, 1.f));
-          c = (double)cf;
-          s = (double)(tf * cf);
+  if constexpr (K > 1) {
+    // H scaled by the power of two that brings its largest diagonal entry to [1, 2)
+    double mx = 0.0;
 #pragma unroll
-          for (int nw = 0; nw < 2; ++nw) {
-            const double f = fma(-0.5, fma(c, c, s * s), 1.5);
-            c *= f;
-            s *= f;
-          }
-        }
-        cs[2 * lane] = c;
-        cs[2 * lane + 1] = s;
-      }
-      __syncwarp();
-      const int slot = lane / K, i = lane % K;
-      int p = 0, q = 0;
-      double c = 1.0, s = 0.0;
-      const bool act = slot < K / 2;
-      if (act) {
-        rr_pair(K, r, slot, &p, &q);
-        c = cs[2 * slot];
-        s = cs[2 * slot + 1];
-      }
-      // columns p, q of H and V: H <- H·J, V <- V·J
-      double hip = 0, hiq = 0, vip = 0, viq = 0;
-      if (act) {
-        hip = H[i * K + p];
-        hiq = H[i * K + q];
-        vip = V[i * K + p];
-        viq = V[i * K + q];
-      }
-      __syncwarp();
-      if (act) {
-        H[i * K + p] = c * hip - s * hiq;
-        H[i * K + q] = s * hip + c * hiq;
-        V[i * K + p] = c * vip - s * viq;
-        V[i * K + q] = s * vip + c * viq;
-      }
-      __syncwarp();
-      // rows p, q: H <- Jᵀ·H
-      double hpi = 0, hqi = 0;
-      if (act) {
-        hpi = H[p * K + i];
-        hqi = H[q * K + i];
-      }
-      __syncwarp();
-      if (act) {
-        H[p * K + i] = c * hpi - s * hqi;
-        H[q * K + i] = s * hpi + c * hqi;
-      }
-      __syncwarp();
+    for (int i = 0; i < K; ++i) mx = fmax(mx, fabs(H[i * K + i]));
+    const int ex = (int)((__double_as_longlong(mx) >> 52) & 0x7ff);
+    const bool scaled = ex > 0 && ex < 2046;  // neither zero nor infinite or NaN
+    const double up = scaled ? __longlong_as_double((long long)(2046 - ex) << 52) : 1.0;
+    const double down = scaled ? __longlong_as_double((long long)ex << 52) : 1.0;
+    __syncwarp();
+    for (int i = lane; i < K * K; i += 32) H[i] *= up;
+    __syncwarp();
+    constexpr int NPR = K / 2;                      // pairs of a round
+    constexpr int NH = NPR * NPR, NVL = K * NPR / 2;  // lanes on H and on V
+    const bool on_h = lane < NH, act = lane < NH + NVL;
+    const int vl = on_h ? 0 : (lane - NH) % NVL;  // (idle lanes repeat one that is not)
+    const int row = vl % K;                          // lanes on V: the row
+    const int sa = on_h ? lane / NPR : 2 * (vl / K) % NPR;
+    const int sb = on_h ? lane % NPR : (2 * (vl / K) + 1) % NPR;
+    // the pairs of slots sa and sb in every round, four bits an index (rounds 0-3, then 4-6)
+    unsigned long long pairs_lo = 0, pairs_hi = 0;
+#pragma unroll
+    for (int r = 0; r < K - 1; ++r) {
+      int pa, qa, pb, qb;
+      rr_pair(K, r, sa, &pa, &qa);
+      rr_pair(K, r, sb, &pb, &qb);
+      const unsigned long long w = (unsigned long long)(pa | qa << 4 | pb << 8 | qb << 12)
+                                   << (16 * (r & 3));
+      if (r < 4)
+        pairs_lo |= w;
+      else
+        pairs_hi |= w;
     }
+#pragma unroll 1
+    for (int sweep = 0; sweep < kJacobiSweeps; ++sweep) {
+      double off = 0.0, dia = 0.0;
+#pragma unroll
+      for (int i = lane; i < K * K; i += 32) {
+        const double h = H[i];
+        if (i / K == i % K)
+          dia += h * h;
+        else
+          off += h * h;
+      }
+      off = warp_sum(off);
+      dia = warp_sum(dia);
+      // off-diagonal entries below ~1e-13 of the matrix: the eigenvalue error left is their
+      // square over the gap (the FP64 rounding floor of `off` is ~K²·eps²·dia, so a tighter test
+      // would never be met and run every sweep); also stops on NaN
+      if (!__any_sync(0xffffffffu, off > 1e-26 * dia)) break;  // (the same in every lane)
+#pragma unroll 1
+      for (int r = 0; r < K - 1; ++r) {
+        const uint32_t pr = (uint32_t)((r < 4 ? pairs_lo : pairs_hi) >> (16 * (r & 3)));
+        const int pa = pr & 15, qa = pr >> 4 & 15, pb = pr >> 8 & 15, qb = pr >> 12 & 15;
+        double* const B = on_h ? H : V;
+        __builtin_assume(__isShared(B));
+        const int i00 = (on_h ? pa * K + pb : row * K + pa), i01 = (on_h ? pa * K + qb : row * K + qa);
+        const int i10 = (on_h ? qa * K + pb : row * K + pb), i11 = (on_h ? qa * K + qb : row * K + qb);
+        const double e00 = B[i00], e01 = B[i01], e10 = B[i10], e11 = B[i11];
+        double ca, sna, cb, snb;
+        jacobi_angle(H[pa * K + pa], H[qa * K + qa], H[pa * K + qa], &ca, &sna);
+        jacobi_angle(H[pb * K + pb], H[qb * K + qb], H[pb * K + qb], &cb, &snb);
+        __syncwarp();
+        // H: columns by pair b, then rows by pair a (Jᵀ·H·J); V: (e00, e01) by pair a, (e10, e11) by
+        // pair b.  Selects, no branch: lanes that part here stay parted for the rounds that follow
+        const double c0 = on_h ? cb : ca, s0 = on_h ? snb : sna;
+        const double cr = on_h ? ca : 1.0, sr = on_h ? sna : 0.0;
+        const double t00 = c0 * e00 - s0 * e01, t01 = s0 * e00 + c0 * e01;
+        const double t10 = cb * e10 - snb * e11, t11 = snb * e10 + cb * e11;
+        if (act) {
+          B[i00] = cr * t00 - sr * t10;
+          B[i01] = cr * t01 - sr * t11;
+          B[i10] = sr * t00 + cr * t10;
+          B[i11] = sr * t01 + cr * t11;
+        }
+        __syncwarp();
+      }
+    }
+    if (lane < K) H[lane * K + lane] *= down;  // (the diagonal is what is read)
+    __syncwarp();
   }
 }
 
@@ -266,8 +331,7 @@ struct Smem {
   static constexpr int vmat = align16(gram + 2 * K * K * 8);             // double V[K*K]
   static constexpr int rinv = align16(vmat + K * K * 8);                 // float Rinv[K*K]
   static constexpr int qv = align16(rinv + K * K * 4);                   // float q[K]
-  static constexpr int cs = align16(qv + K * 4);                         // double cs[kMaxK]
-  static constexpr int ritz = align16(cs + kMaxK * 8);                   // double θ[K], λ
+  static constexpr int ritz = align16(qv + K * 4);                       // double θ[K], λ
   static constexpr int ctl = align16(ritz + (kMaxK + 1) * 8);            // int [4]
   static constexpr int tbar = align16(ctl + 16);  // uint64 [kWarps][2]: tensor-core tile copies
   static constexpr int xs = align16(tbar + kWarps * 2 * 8);              // float X[K][kMaxRows]
@@ -280,7 +344,7 @@ struct Smem {
   static constexpr int region = TC ? align1024(xs + xs_bytes) : align16(xs + xs_bytes);
   static constexpr int yred = region;                                    // float [4*kThreads][K]
   static constexpr int hist = align16(yred + 4 * kThreads * K * 4);      // uint32 [kMaxCols]
-  static constexpr int xrow = hist;  // tensor-core kernel, a matrix multiplied as C·X: X as [row][v]
+  static constexpr int xrow = hist;  // tensor-core kernel, a matrix multiplied as C·X: X by row (yq)
   static constexpr int region_bytes =
       TC ? cmax(2 * kTcStageFloats * 4, 4 * kThreads * K * 4)
          : cmax(hist + kMaxCols * 4 - region, kRingBytes);
@@ -291,7 +355,7 @@ struct Smem {
   static constexpr int scan = align16(lw + kMaxPicks * 4);             // uint32 [40], double[32]
   static constexpr int svr = align16(scan + 40 * 4 + 32 * 8);           // float S[K*K] (VR)
   static constexpr int total_amm = align16(svr + K * K * 4);
-  static_assert(gpart % 8 == 0 && cs % 8 == 0 && xs % 16 == 0 && region % 16 == 0,
+  static_assert(gpart % 8 == 0 && ritz % 8 == 0 && xs % 16 == 0 && region % 16 == 0,
                 "shared-memory alignment");
   static_assert(!TC || xrow + kMaxRows * K * 4 <= region + region_bytes, "X by row fits the region");
   static_assert(!TC || total <= 227 * 1024, "the tensor-core layout exceeds a CTA's shared memory");
@@ -345,112 +409,113 @@ __device__ __forceinline__ float team_allreduce(float (&d)[NV], float* part, int
 // (rank-deficient block or a non-finite λ); ctl[2]: a Ritz pair was formed.
 template <int K>
 __device__ __noinline__ void ritz_step(const Args& a, int mi, int it, double* Gm, double* Hm,
-                                       double* Vm, double* cs, double* ritz, float* Rinv,
-                                       float* qv, int* ctl, double* scratch, int lane,
-                                       bool writer, bool force_rr) {
+                                       double* Vm, double* ritz, float* Rinv, float* qv, int* ctl,
+                                       double* scratch, int lane, bool writer, bool force_rr) {
+  __builtin_assume(__isShared(Gm));
+  __builtin_assume(__isShared(Hm));
+  __builtin_assume(__isShared(Vm));
+  __builtin_assume(__isShared(scratch));
+  __builtin_assume(__isShared(ritz));
+  __builtin_assume(__isShared(Rinv));
   const bool first = (it == 0);
   const bool rr = !first && ((K == 1) || ((it % a.rr_period) == 0) || (it >= a.max_iter) ||
                              force_rr);
-  if (rr) jacobi_warp<K>(Hm, Vm, cs, lane);
-  // the Ritz values (lane 0: K entries)
+  if (rr) jacobi_warp<K>(Hm, Vm, lane);
+  // the Ritz values, descending: lane i < K places its own by its rank (ties in index order); the
+  // first of the largest gives λ and its vector
   int st = 0;
-  if (lane == 0) {
-    ctl[2] = rr ? 1 : 0;
-    if (rr) {
-      int best = 0;
-      for (int i = 1; i < K; ++i)
-        if (Hm[i * K + i] > Hm[best * K + best]) best = i;
-      const double lam = Hm[best * K + best];
-      for (int i = 0; i < K; ++i) qv[i] = (float)Vm[i * K + best];
-      double th[kMaxK];  // Ritz values, descending
-      for (int i = 0; i < K; ++i) th[i] = Hm[i * K + i];
-      for (int i = 0; i < K; ++i)
-        for (int j = i + 1; j < K; ++j)
-          if (th[j] > th[i]) {
-            const double tmp = th[i];
-            th[i] = th[j];
-            th[j] = tmp;
-          }
-      for (int i = 0; i < K; ++i) ritz[i] = th[i];
-      ritz[kMaxK] = lam;
-      if (!isfinite(lam)) st = 2;
+  if (rr) {
+    double mine = lane < K ? Hm[lane * K + lane] : 0.0;
+    int rank = 0;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const double o = __shfl_sync(0xffffffffu, mine, j);
+      rank += (o > mine || (o == mine && j < lane)) ? 1 : 0;
     }
+    // (a NaN ranks against nothing: such a block is reported below, whatever its order)
+    if (!isfinite(mine)) rank = lane < K ? lane : 0;
+    const uint32_t top = __ballot_sync(0xffffffffu, lane < K && rank == 0);
+    const int best = top ? __ffs(top) - 1 : 0;
+    const double lam = __shfl_sync(0xffffffffu, mine, best);
+    if (lane < K) {
+      ritz[rank] = mine;
+      qv[lane] = (float)Vm[lane * K + best];
+    }
+    if (lane == 0) ritz[kMaxK] = lam;
+    if (__any_sync(0xffffffffu, lane < K && !isfinite(mine))) st = 2;
   }
-  st = __shfl_sync(0xffffffffu, st, 0);
-  // The next basis, by the whole warp with the K x K matrices in shared memory (`scratch`:
-  // 4·K² doubles); each entry is summed in the same order as a sequential loop would.
+  if (lane == 0) ctl[2] = rr ? 1 : 0;
+  // The next basis, by the whole warp; each entry is summed in the order of a sequential loop.
   double* Gp = scratch;              // VᵀGV (or G)
   double* T = scratch + K * K;       // G·V
-  double* L = scratch + 2 * K * K;   // Cholesky factor (lower)
   double* Li = scratch + 3 * K * K;  // L⁻¹ (lower)
   if (st == 0) {
     if (rr) {
+#pragma unroll
       for (int idx = lane; idx < K * K; idx += 32) {
         const int i = idx / K, j = idx % K;
         double acc = 0.0;
+#pragma unroll
         for (int k = 0; k < K; ++k) acc += Gm[i * K + k] * Vm[k * K + j];
         T[idx] = acc;
       }
       __syncwarp();
+#pragma unroll
       for (int idx = lane; idx < K * K; idx += 32) {
         const int i = idx / K, j = idx % K;
         double acc = 0.0;
+#pragma unroll
         for (int k = 0; k < K; ++k) acc += Vm[k * K + i] * T[k * K + j];
         Gp[idx] = acc;
       }
     } else {
       for (int idx = lane; idx < K * K; idx += 32) Gp[idx] = Gm[idx];
     }
-    for (int idx = lane; idx < K * K; idx += 32) L[idx] = 0.0;
     __syncwarp();
     double tr = 0.0;
+#pragma unroll
     for (int i = 0; i < K; ++i) tr += Gp[i * K + i];
     bool ok = tr > 0.0 && isfinite(tr);
-    // Cholesky, column by column: the diagonal by lane 0, the column below it by lanes j+1..;
-    // one reciprocal square root per column gives both L_jj = d·d^(-1/2) and 1/L_jj (kept in
-    // Ri, which takes T's place: T is dead once Gp is formed), so no step divides
-    double* Ri = T;
-    for (int j = 0; j < K && ok; ++j) {
-      if (lane == 0) {
-        double d = Gp[j * K + j];
-        for (int k = 0; k < j; ++k) d -= L[j * K + k] * L[j * K + k];
-        const bool good = d > 1e-24 * tr;
-        const double r = good ? rsqrt(d) : 0.0;
-        L[j * K + j] = good ? d * r : 0.0;
-        Ri[j] = r;
-        cs[0] = good ? 1.0 : 0.0;
-      }
-      __syncwarp();
-      ok = cs[0] != 0.0;
-      if (ok && lane > j && lane < K) {
-        const int i = lane;
-        double sv = Gp[i * K + j];
-        for (int k = 0; k < j; ++k) sv -= L[i * K + k] * L[j * K + k];
-        L[i * K + j] = sv * Ri[j];
-      }
-      __syncwarp();
+    // Cholesky L·Lᵀ = Gp in registers, lane i < K holding row i: per column one reciprocal square root
+    // gives both L_jj = d·d^(-1/2) and 1/L_jj, so no step divides
+    double l[K], ri[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) l[k] = lane < K ? Gp[lane * K + k] : 0.0;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const double d = __shfl_sync(0xffffffffu, l[j], j);
+      const bool good = d > 1e-24 * tr;
+      ok = ok && good;
+      ri[j] = good ? rsqrt(d) : 0.0;
+      l[j] = l[j] * ri[j];
+#pragma unroll
+      for (int k = j + 1; k < K; ++k) l[k] -= l[j] * __shfl_sync(0xffffffffu, l[j], k);
     }
     if (!ok) {  // rank-deficient block: no result for this matrix
       st = 2;
     } else {
       // L⁻¹, column j by lane j (forward substitution)
+      double x[K];
+#pragma unroll
+      for (int i = 0; i < K; ++i) {
+        double sv = 0.0;
+#pragma unroll
+        for (int k = 0; k < i; ++k) sv += __shfl_sync(0xffffffffu, l[k], i) * x[k];
+        x[i] = i < lane ? 0.0 : i == lane ? ri[i] : -sv * ri[i];
+      }
       if (lane < K) {
-        const int j = lane;
-        for (int i = 0; i < K; ++i) Li[i * K + j] = 0.0;
-        Li[j * K + j] = Ri[j];
-        for (int i = j + 1; i < K; ++i) {
-          double sv = 0.0;
-          for (int k = j; k < i; ++k) sv += L[i * K + k] * Li[k * K + j];
-          Li[i * K + j] = -sv * Ri[i];
-        }
+#pragma unroll
+        for (int i = 0; i < K; ++i) Li[i * K + lane] = x[i];
       }
       __syncwarp();
-      // M = V·L⁻ᵀ (or L⁻ᵀ without a rotation); (L⁻ᵀ)[k][j] = Li[j][k] for k <= j
+      // M = V·L⁻ᵀ (or L⁻ᵀ without a rotation); (L⁻ᵀ)[k][j] = Li[j][k], zero for k > j
+#pragma unroll
       for (int idx = lane; idx < K * K; idx += 32) {
         const int i = idx / K, j = idx % K;
         double sv = 0.0;
         if (rr) {
-          for (int k = 0; k <= j; ++k) sv += Vm[i * K + k] * Li[j * K + k];
+#pragma unroll
+          for (int k = 0; k < K; ++k) sv += Vm[i * K + k] * Li[j * K + k];
         } else {
           sv = (i <= j) ? Li[j * K + i] : 0.0;
         }
@@ -471,20 +536,62 @@ __device__ __noinline__ void ritz_step(const Args& a, int mi, int it, double* Gm
 // ---- variance reduction helpers, out of line so that their registers do not compete with the
 // product loop's ----
 // S = X_memoᵀ·X (FP64 sums over team 0's rows, into Svr) and D = X − X_memo·S in place of X
-// (X saved to Xsave, [row][v], restored by vr_add_memo after the product); called by every
-// thread of the CTA.
+// (X saved to Xsave, restored by vr_add_memo after the product); called by every thread of the CTA.
+// The memo slots hold a thread's 4 rows as K float4s, float4 i of thread t at i·kThreads + t: every
+// access is coalesced, and every thread reads back only what it wrote.  For 8 vectors S is formed
+// on the FP64 tensor cores from a copy of X_memo in shared memory (`Ys`), as the Gram matrices are.
 template <int K>
-__device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xsave,
+__device__ __forceinline__ void memo_load(const float* p, int t, float (&v)[4][K]) {
+#pragma unroll
+  for (int i = 0; i < K; ++i) {
+    const float4 q = reinterpret_cast<const float4*>(p)[i * kThreads + t];
+    const float w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[(4 * i + c) / K][(4 * i + c) % K] = w[c];
+  }
+}
+template <int K>
+__device__ __forceinline__ void memo_store(float* p, int t, const float (&v)[4][K]) {
+#pragma unroll
+  for (int i = 0; i < K; ++i)
+    reinterpret_cast<float4*>(p)[i * kThreads + t] =
+        make_float4(v[4 * i / K][4 * i % K], v[(4 * i + 1) / K][(4 * i + 1) % K],
+                    v[(4 * i + 2) / K][(4 * i + 2) % K], v[(4 * i + 3) / K][(4 * i + 3) % K]);
+}
+__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b);
+
+template <int K>
+__device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xsave, float* Ys,
                                            double* gpart, float* Svr, int P, int r0, int t,
                                            int warp, int lane, int team) {
   const int tw = P / 32;  // warps of team 0
-  if (warp < tw) {
+  float xm[4][K];
+  if (team == 0) memo_load<K>(Xm, t, xm);
+  if constexpr (K == 8) {
+    if (team == 0) {  // warp-uniform
+      y_store<K>(Ys, t, xm);
+      __syncwarp();
+      double d[2] = {0.0, 0.0};
+      const int g = lane >> 2, tq = lane & 3, rb = 128 * warp;
+#pragma unroll 4
+      for (int k = 0; k < 32; ++k) {
+        const int row = rb + 4 * k + tq;
+        mma_f64(d, (double)Ys[yat<K>(row, g)], (double)Xs[xs_idx<K>(g, row)]);
+      }
+      gpart[warp * K * K + g * K + 2 * tq] = d[0];
+      gpart[warp * K * K + g * K + 2 * tq + 1] = d[1];
+    }
+  } else if (warp < tw) {
     for (int ab = 0; ab < K * K; ++ab) {
       const int va = ab / K, vb = ab % K;
       double sv = 0.0;
 #pragma unroll
-      for (int e = 0; e < 4; ++e)
-        sv = fma((double)Xm[(r0 + e) * K + va], (double)Xs[xs_idx<K>(vb, r0 + e)], sv);
+      for (int e = 0; e < 4; ++e) {
+        float x = 0.f;
+#pragma unroll
+        for (int v = 0; v < K; ++v) x = v == va ? xm[e][v] : x;
+        sv = fma((double)x, (double)Xs[xs_idx<K>(vb, r0 + e)], sv);
+      }
       sv = warp_sum(sv);
       if (lane == 0) gpart[warp * K * K + ab] = sv;
     }
@@ -497,16 +604,22 @@ __device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xs
   }
   __syncthreads();
   if (team == 0) {
-    for (int e = 0; e < 4; ++e) {
-      float xm[K];
+    float x[4][K];
 #pragma unroll
-      for (int v = 0; v < K; ++v) xm[v] = Xm[(r0 + e) * K + v];
+    for (int e = 0; e < 4; ++e)
 #pragma unroll
-      for (int vb = 0; vb < K; ++vb) {
-        float d = Xs[xs_idx<K>(vb, r0 + e)];
-        Xsave[(r0 + e) * K + vb] = d;
+      for (int vb = 0; vb < K; ++vb) x[e][vb] = Xs[xs_idx<K>(vb, r0 + e)];
+    memo_store<K>(Xsave, t, x);
 #pragma unroll
-        for (int va = 0; va < K; ++va) d = fmaf(-xm[va], Svr[va * K + vb], d);
+    for (int vb = 0; vb < K; ++vb) {
+      float sc[K];
+#pragma unroll
+      for (int va = 0; va < K; ++va) sc[va] = Svr[va * K + vb];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float d = x[e][vb];
+#pragma unroll
+        for (int va = 0; va < K; ++va) d = fmaf(-xm[e][va], sc[va], d);
         Xs[xs_idx<K>(vb, r0 + e)] = d;  // this thread alone reads and writes its rows here
       }
     }
@@ -514,37 +627,44 @@ __device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xs
   __syncthreads();
 }
 
-// Y += Y_memo·S over this thread's rows, and X back in place of D (team 0, once no team
-// multiplies any more).
+// Y += Y_memo·S over this thread's rows (Y at Yp, laid out as the memo slots), and X back in place of
+// D (team 0, once no team multiplies any more).
 template <int K>
-__device__ __noinline__ void vr_add_memo(float (&Y)[4][K], const float* Ym, const float* Svr,
-                                         const float* Xsave, float* Xs, int r0) {
-  for (int e = 0; e < 4; ++e) {
+__device__ __noinline__ void vr_add_memo(float* Yp, const float* Ym, const float* Svr,
+                                         const float* Xsave, float* Xs, int r0, int t) {
+  float v4[4][K], Y[4][K];
+  memo_load<K>(Xsave, t, v4);
 #pragma unroll
-    for (int v = 0; v < K; ++v) Xs[xs_idx<K>(v, r0 + e)] = Xsave[(r0 + e) * K + v];
-    float ym[K];
+  for (int e = 0; e < 4; ++e)
 #pragma unroll
-    for (int v = 0; v < K; ++v) ym[v] = Ym[(r0 + e) * K + v];
+    for (int v = 0; v < K; ++v) Xs[xs_idx<K>(v, r0 + e)] = v4[e][v];
+  memo_load<K>(Ym, t, v4);
+  memo_load<K>(Yp, t, Y);
 #pragma unroll
-    for (int vb = 0; vb < K; ++vb) {
+  for (int vb = 0; vb < K; ++vb) {
+    float sc[K];
+#pragma unroll
+    for (int va = 0; va < K; ++va) sc[va] = Svr[va * K + vb];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
       float acc = Y[e][vb];
 #pragma unroll
-      for (int va = 0; va < K; ++va) acc = fmaf(ym[va], Svr[va * K + vb], acc);
+      for (int va = 0; va < K; ++va) acc = fmaf(v4[e][va], sc[va], acc);
       Y[e][vb] = acc;
     }
   }
+  memo_store<K>(Yp, t, Y);
 }
 
-// The memo pair (X_memo, Y_memo) <- (X, Y) over this thread's rows (team 0).
+// X_memo <- X over this thread's rows (team 0).
 template <int K>
-__device__ __noinline__ void vr_store_memo(const float (&Y)[4][K], float* Xm, float* Ym,
-                                           const float* Xs, int r0) {
+__device__ __noinline__ void vr_store_memo(float* Xm, const float* Xs, int r0, int t) {
+  float x[4][K];
+#pragma unroll
   for (int e = 0; e < 4; ++e)
 #pragma unroll
-    for (int v = 0; v < K; ++v) {
-      Xm[(r0 + e) * K + v] = Xs[xs_idx<K>(v, r0 + e)];
-      Ym[(r0 + e) * K + v] = Y[e][v];
-    }
+    for (int v = 0; v < K; ++v) x[e][v] = Xs[xs_idx<K>(v, r0 + e)];
+  memo_store<K>(Xm, t, x);
 }
 
 // One FP64 tensor-core product D += A·B (m8n8k4, FP64 accumulation), fragments as in the PTX
@@ -556,7 +676,7 @@ __device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b) {
 }
 
 // Gram matrices of the block, G = YᵀY and H = sym(XᵀY), in FP64 over team 0's rows (the only
-// team holding the summed Y, here in shared memory as Ys[row][v]); called by every thread of the
+// team holding the summed Y, here in shared memory as Ys, see yq); called by every thread of the
 // CTA.  For 8 vectors each warp of team 0 multiplies its 128 rows on the FP64 tensor cores: per
 // 4 rows one m8n8k4 product for G (A = Yᵀ, B = Y: lane 4·g + t supplies Y[row t][vector g] to
 // both) and one for XᵀY (A = Xᵀ); FP32 × FP32 products are exact in FP64.  For fewer vectors
@@ -579,7 +699,7 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 #pragma unroll 4
       for (int k = 0; k < 32; ++k) {
         const int row = rb + 4 * k + tq;
-        const double y = (double)Ys[row * K + g];
+        const double y = (double)Ys[yat<K>(row, g)];
         const double x = (double)Xs[xs_idx<K, TC>(g, row)];
         mma_f64(dg, y, y);
         mma_f64(dh, x, y);
@@ -623,7 +743,7 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 #pragma unroll
       for (int e = 0; e < 4; ++e)
 #pragma unroll
-        for (int v = 0; v < K; ++v) y[e][v] = Ys[(r0 + e) * K + v];
+        for (int v = 0; v < K; ++v) y[e][v] = Ys[yat<K>(r0 + e, v)];
 #pragma unroll
       for (int bt = 0; bt < NB; ++bt) {
         double d[8];
@@ -678,7 +798,7 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 
 // Y = C·X over this team's share of C's columns (C = A·Aᵀ, ldc x ldc, zeros past m), this thread's
 // rows r0 .. r0 + 3, for an even number of vectors: per column one 16-byte load of C (coalesced
-// over the team, four columns ahead in registers) against X's row (broadcast loads: `xrow` [row][v],
+// over the team, four columns ahead in registers) against X's row (broadcast loads: `xrow`, see yq,
 // or without it the interleaved pairs of Xs), in packed FP32 FMAs.  Bounded by the FMAs and by an
 // SM's share of the L2 (16 packed FMAs per 16 bytes).  The sums are taken in runs of 16 columns, added
 // up in this thread's slot of shared memory (`slots`, [value / 4][thread]): one FP32 chain over a
@@ -687,8 +807,8 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 // registers do not compete with the other product loops'.
 template <int K>
 __device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, const float* xrow,
-                                        const float* Xs, float4* slots, int r0, int g0, int gstep,
-                                        float (&Y)[4][K]) {
+                                        const float* Xs, float4* slots, int r0, int g0,
+                                        int gstep) {
   constexpr int KP = K / 2;
   float2 run[4][KP];
 #pragma unroll
@@ -731,7 +851,7 @@ __device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, co
         if (xrow) {
 #pragma unroll
           for (int p = 0; p < KP; p += 2) {
-            const float4 v = *reinterpret_cast<const float4*>(xrow + k * K + 2 * p);
+            const float4 v = reinterpret_cast<const float4*>(xrow)[yq<K>(g, j * (K / 4) + p / 2)];
             x[p] = make_float2(v.x, v.y);
             x[p + 1] = make_float2(v.z, v.w);
           }
@@ -767,10 +887,9 @@ __device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, co
 #pragma unroll
   for (int e = 0; e < 4; ++e)
 #pragma unroll
-    for (int p = 0; p < KP; ++p) {
-      Y[e][2 * p] = run[e][p].x;
-      Y[e][2 * p + 1] = run[e][p].y;
-    }
+    for (int p = 0; p < KP; p += 2)
+      slot[(e * KP + p) / 2 * kThreads] =
+          make_float4(run[e][p].x, run[e][p].y, run[e][p + 1].x, run[e][p + 1].y);
 }
 
 template <int K, int GC, bool TC = false>
@@ -789,7 +908,6 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
   double* Vm = reinterpret_cast<double*>(smem + SL::vmat);
   float* Rinv = reinterpret_cast<float*>(smem + SL::rinv);
   float* qv = reinterpret_cast<float*>(smem + SL::qv);
-  double* cs = reinterpret_cast<double*>(smem + SL::cs);
   double* ritz = reinterpret_cast<double*>(smem + SL::ritz);
   int* ctl = reinterpret_cast<int*>(smem + SL::ctl);
   float* Xs = reinterpret_cast<float*>(smem + SL::xs);  // X, one copy for all teams: [v][row]
@@ -969,26 +1087,16 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
     for (;; ++it) {
       // ---- Gram matrices of the block: G = YᵀY, H = sym(XᵀY) (FP64, team 0's rows), from a
       // shared-memory copy of team 0's Y (each thread reads back only its own rows) ----
-      if (team == 0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-          for (int v = 0; v < K; ++v) yred[(r0 + e) * K + v] = Y[e][v];
-      }
+      if (team == 0) y_store<K>(yred, t, Y);
       gram_step<K, TC>(Xs, yred, gpart, Gm, Hm, P, r0, t, warp, lane, team);
       // (gpart, summed into Gm and Hm above, is the Ritz step's scratch)
       if (warp == 0)
-        ritz_step<K>(a, mi, it, Gm, Hm, Vm, cs, ritz, Rinv, qv, ctl, gpart, lane, writer,
+        ritz_step<K>(a, mi, it, Gm, Hm, Vm, ritz, Rinv, qv, ctl, gpart, lane, writer,
                      vr && prev_exact);
       __syncthreads();
       // team 0's Y back from its shared-memory copy (not held in registers across the two
       // out-of-line steps, which then get the registers for themselves)
-      if (team == 0) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-          for (int v = 0; v < K; ++v) Y[e][v] = yred[(r0 + e) * K + v];
-      }
+      if (team == 0) y_load<K, false>(yred, t, Y);
       if (ctl[2] && ctl[1] == 0) {
         // residual of the top Ritz pair, r = C·v − λ·v = (Y − λ·X)·q, over team 0's rows (FP64)
         const double lam = ritz[kMaxK];
@@ -1042,23 +1150,35 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       }
       // ---- X <- Y·M (team 0 writes the shared copy) ----
       if (team == 0) {
+        float X[4][K];
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-          float xj[4];
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             float s = 0.f;
 #pragma unroll
             for (int i = 0; i < K; ++i) s = fmaf(Y[e][i], Rinv[i * K + j], s);
-            xj[e] = s;
+            X[e][j] = s;
           }
+        }
+        if constexpr (TC) {  // [v][row]; and by row for a product with C (in the idle tile region)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) Xs[xs_idx<K, TC>(j, r0 + e)] = xj[e];
-          if (TC && M.C) {  // X by row for the product with C (in the idle tile region)
-            float* xr = reinterpret_cast<float*>(smem + SL::xrow);
+          for (int j = 0; j < K; ++j)
+            *reinterpret_cast<float4*>(Xs + xs_idx<K, true>(j, r0)) =
+                make_float4(X[0][j], X[1][j], X[2][j], X[3][j]);
+          if (M.C) y_store<K>(reinterpret_cast<float*>(smem + SL::xrow), t, X);
+        } else if constexpr (K % 2 == 0) {  // interleaved pairs
 #pragma unroll
-            for (int e = 0; e < 4; ++e) xr[(r0 + e) * K + j] = xj[e];
-          }
+          for (int j = 0; j < K; j += 2)
+#pragma unroll
+            for (int e = 0; e < 4; e += 2)
+              *reinterpret_cast<float4*>(Xs + xs_idx<K>(j, r0 + e)) =
+                  make_float4(X[e][j], X[e][j + 1], X[e + 1][j], X[e + 1][j + 1]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < K; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) Xs[xs_idx<K, TC>(j, r0 + e)] = X[e][j];
         }
       }
       __syncthreads();
@@ -1131,16 +1251,21 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // the sampled product multiplies, D = X − X_memo·S, in place of X; Y_memo·S is added,
       // and X put back, once the product is summed ----
       const bool use_d = wamm && memo;
-      if (use_d) vr_difference<K>(Xm, Xs, Xsave, gpart, Svr, P, r0, t, warp, lane, team);
+      if (use_d) vr_difference<K>(Xm, Xs, Xsave, yred, gpart, Svr, P, r0, t, warp, lane, team);
       const float* Xsrc = Xs;  // X, or D in its place
       // ---- Y = C·X (or its AMM estimate): the fused pass over the columns (team-local) ----
       const bool rows = r0 < m;
       int buf = 0;
       const bool by_c = K % 2 == 0 && M.C != nullptr && !wamm;  // an exact product as C·X
       if (by_c) {
-        if constexpr (K % 2 == 0)
+        // (nothing that this kernel keeps in registers is passed to an out-of-line function by
+        // address: it would live in local memory, and the L1 left beside the shared memory is
+        // streamed through by the products)
+        if constexpr (K % 2 == 0) {
           cx_product<K>(M.C, M.ldc, TC ? reinterpret_cast<const float*>(smem + SL::xrow) : nullptr,
-                        Xs, reinterpret_cast<float4*>(yred), r0, gteam, NTG, Y);
+                        Xs, reinterpret_cast<float4*>(yred), r0, gteam, NTG);
+          memo_load<K>(yred, t, Y);
+        }
         __syncthreads();  // the slots lie where Y is copied next
       } else if constexpr (TC) {
         // ---- tensor-core pass (exact mode, 8 vectors).  Warp wi of a team owns the team's
@@ -1278,8 +1403,9 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
         for (int i = 0; i < 8; ++i) {
           if (i >= nblk) break;
           const int row = team * 4 * P + rbase + 16 * i + g;
-          *reinterpret_cast<float2*>(yred + row * K + 2 * tq) = make_float2(yacc[i][0], yacc[i][1]);
-          *reinterpret_cast<float2*>(yred + (row + 8) * K + 2 * tq) =
+          *reinterpret_cast<float2*>(yred + yat<K>(row, 2 * tq)) =
+              make_float2(yacc[i][0], yacc[i][1]);
+          *reinterpret_cast<float2*>(yred + yat<K>(row + 8, 2 * tq)) =
               make_float2(yacc[i][2], yacc[i][3]);
         }
         __syncthreads();
@@ -1287,12 +1413,11 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
 #pragma unroll
           for (int e = 0; e < 4; ++e)
 #pragma unroll
-            for (int v = 0; v < K; ++v) {
-              float s = 0.f;
-              if (rows)
-                for (int tm = 0; tm < NT; ++tm) s += yred[((tm * 4 * P) + r0 + e) * K + v];
-              Y[e][v] = s;
-            }
+            for (int v = 0; v < K; ++v) Y[e][v] = 0.f;
+          if (rows) {
+#pragma unroll 1
+            for (int tm = 0; tm < NT; ++tm) y_load<K, true>(yred, tm * P + t, Y);
+          }
         }
       } else {
 #pragma unroll
@@ -1417,45 +1542,27 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // ---- sum the team partials of Y (fixed order), every team receives the total ----
       if ((!TC || by_c) && NT > 1) {
         __syncthreads();
-        if (rows) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int v = 0; v < K; ++v) yred[((team * 4 * P) + r0 + e) * K + v] = Y[e][v];
-        }
+        if (rows && team > 0) y_store<K>(yred, t, Y);  // (slot team·P + tl)
         __syncthreads();
         if (rows && team == 0) {  // only team 0 uses the summed Y (Gram, residual, X, v)
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int v = 0; v < K; ++v) {
-              float s = 0.f;
-              for (int tm = 0; tm < NT; ++tm) s += yred[((tm * 4 * P) + r0 + e) * K + v];
-              Y[e][v] = s;
-            }
+#pragma unroll 1
+          for (int tm = 1; tm < NT; ++tm) y_load<K, true>(yred, tm * P + t, Y);
         }
       }
       // ---- sum the CTA partials of the cluster through distributed shared memory (fixed
       // rank order): every CTA receives the same Y ----
       if (CL > 1) {
         __syncthreads();
-        if (team == 0 && rows) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int v = 0; v < K; ++v) yred[(r0 + e) * K + v] = Y[e][v];
-        }
+        if (team == 0 && rows) y_store<K>(yred, t, Y);
         cluster.sync();
         if (rows && team == 0) {
 #pragma unroll
           for (int e = 0; e < 4; ++e)
 #pragma unroll
-            for (int v = 0; v < K; ++v) {
-              float s = 0.f;
-              for (int rk = 0; rk < CL; ++rk)
-                s += *cluster.map_shared_rank(&yred[(r0 + e) * K + v], rk);
-              Y[e][v] = s;
-            }
+            for (int v = 0; v < K; ++v) Y[e][v] = 0.f;
+#pragma unroll 1
+          for (int rk = 0; rk < CL; ++rk)
+            y_load<K, true>(cluster.map_shared_rank(yred, rk), t, Y);
         }
         cluster.sync();  // the buffers are rewritten by the next step
       }
@@ -1464,10 +1571,19 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       if (use_d) {
         // no team reads X or D any more: every team passed a barrier after its product pass
         // (team sums, cluster sums) or team 0 is the only team
-        if (team == 0) vr_add_memo<K>(Y, Ym, Svr, Xsave, Xs, r0);
+        __syncthreads();  // (the sums' slots are read; below: before Y is copied over these)
+        if (team == 0) {
+          memo_store<K>(yred, t, Y);  // (this thread's own words)
+          vr_add_memo<K>(yred, Ym, Svr, Xsave, Xs, r0, t);
+          memo_load<K>(yred, t, Y);
+        }
+        __syncthreads();
       }
       if (vr && exact_p) {
-        if (team == 0) vr_store_memo<K>(Y, Xm, Ym, Xs, r0);
+        if (team == 0) {
+          memo_store<K>(Ym, t, Y);
+          vr_store_memo<K>(Xm, Xs, r0, t);
+        }
         memo = true;
       }
       prev_exact = exact_p;
