@@ -59,3 +59,27 @@ def test_step_kernel_shapes(m, n, c, dtype, method, kw):
     ctx.power_method(method, torch.from_numpy(x0).cuda())
     assert np.array_equal(ctx.trace()["eigs"], tr["eigs"])
     ctx.close()
+
+
+@pytest.mark.parametrize("step", [40, 1700])
+def test_trace_region_of_any_length(step):
+    """A trace short enough for one copy and one that is copied piece by piece (1700 steps, stopped
+    early by the tolerance) hold the same entries."""
+    from eigenvaluecomputation_by_amm_b200 import AMMContext, column_major
+    m, n, c = 256, 700, 90
+    A = scaled_gaussian(m, n, seed=31)
+    ctx = AMMContext(m, n, c=c, step=step, tol=1e-5, vr_period=4)
+    ctx.set_matrix(column_major(torch.from_numpy(A).cuda()))
+    st = states(c, 32)
+    ctx.set_rng_state(torch.from_numpy(st.view(np.int32)).cuda())
+    x0 = np.random.default_rng(33).standard_normal(m).astype(np.float32)
+    ctx.power_method("exact", torch.from_numpy(x0).cuda())
+    tr = ctx.trace()
+    ref = O.power_method(A, x0, method="exact", step=40, c=c, states=st, vr_period=4)
+    k = tr["steps_run"]
+    assert 1 < k < 40
+    for key in ("eigs", "errs", "coss", "distinct", "t_ns", "kinds"):
+        assert len(tr[key]) == k
+    assert np.all(rel(tr["eigs"], ref.eigs[:k]) < RTOL_LAMBDA_F32)
+    assert np.all(np.diff(tr["t_ns"]) > 0) and set(tr["distinct"]) == {n}
+    ctx.close()
