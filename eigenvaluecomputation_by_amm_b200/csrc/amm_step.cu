@@ -32,7 +32,12 @@
 // and 9.1 us with 1, 4 and 8).
 // No packet is overwritten early: a CTA writes partials of step i + 1 after it has read all
 // packets of y_i, each written by a CTA that had read all its partials of step i; and packets of
-// y_{i+1} are written after all partials of step i + 1, whose writers had read all of y_i.
+// y_{i+1} are written after all partials of step i + 1, whose writers had read all of y_i.  The
+// CTAs' scalars and shares have two places each, by step parity: a CTA that owns no packet (there
+// are fewer packets than CTAs, or fewer owners) waits for no partial, so it may write its shares
+// of step i + 1 before a slow CTA has read those of step i, and the scalars of a step may be
+// rewritten before it has read them; two steps on, it has finished step i, for it wrote the partials
+// of step i + 1 that the packets of y_{i+1} took.
 //
 // What bounds it: large steps the column stream (HBM); small ones the two trips through L2
 // (write, poll: 0.5-0.7 us each from SM to SM) and the CTA-wide reductions between them.
@@ -164,11 +169,11 @@ __host__ __device__ inline int step_packets(const PanelGeom& g) {
 __host__ __device__ inline int step_owned_max(const PanelGeom& g) {
   return (step_packets(g) + g.grid - 1) / g.grid;
 }
-// A CTA's block of y packets: its packets, then per owner warp the shares of x·y, y·y and y·v*; whole
-// 128-byte lines, so that no line has two writers
+// A CTA's block of y packets: its packets, then by step parity and owner warp the shares of x·y, y·y
+// and y·v*; whole 128-byte lines, so that no line has two writers
 constexpr int kShareWarps = 2;
 __host__ __device__ inline int step_block(const PanelGeom& g) {
-  return (step_owned_max(g) + 3 * kShareWarps + 7) / 8 * 8;
+  return (step_owned_max(g) + 2 * 3 * kShareWarps + 7) / 8 * 8;
 }
 
 __host__ __device__ inline StepLayout step_layout(const PanelGeom& g) {
@@ -204,7 +209,7 @@ __host__ __device__ inline StepLayout step_layout(const PanelGeom& g) {
 }
 
 int step_smem(const PanelGeom& g) { return step_layout(g).total; }
-int64_t step_partial_packets(const PanelGeom& g) { return step_packets(g) + 1; }
+int64_t step_partial_packets(const PanelGeom& g) { return step_packets(g) + 2; }
 // y by owners' blocks
 int64_t step_y_packets(const PanelGeom& g) { return (int64_t)step_block(g) * g.grid; }
 // The packet exchange wants enough CTAs that one thread per owned packet is left; a device (or a
@@ -362,8 +367,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     o[9] = row >= 0 ? __ldcg(b.v + row) : 0.f;
     o[12] = row >= 0 ? __ldcg(b.z + row) : 0.f;
   }
-  uint4* const ll1 = b.pk_part;                              // [G][NPT + 1]
-  const size_t ll1_stride = (size_t)NPT + 1;
+  uint4* const ll1 = b.pk_part;                              // [G][NPT + 2]
+  const size_t ll1_stride = (size_t)NPT + 2;
   // x_memo of this thread's rows: the context's copy until the launch's first variance-reduction
   // step, then this CTA's own (each thread reads back what it wrote)
   auto xm_at = [&](int memo) -> float* {
@@ -828,7 +833,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
                      3 * k + 2 < NV ? val(yacc, 3 * k + 2 < NV ? 3 * k + 2 : 0) : 0.f, ep);
       if (t == 0) {
         const double zd = centred ? zdx_s : 0.0;
-        packet_store(out + NPT, sacc, __int_as_float(__double2loint(zd)),
+        packet_store(out + NPT + (i & 1), sacc, __int_as_float(__double2loint(zd)),
                      __int_as_float(__double2hiint(zd)), ep);
       }
     }
@@ -878,7 +883,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
       for (int j = lane; j < G && ok; j += 32 * U) {
         uint4 v[U];
         const int cnt = (G - j + 31) / 32;
-        ok = packets_wait<U>(ll1 + (size_t)j * ll1_stride + NPT, 32 * ll1_stride, cnt, ep, v);
+        ok = packets_wait<U>(ll1 + (size_t)j * ll1_stride + NPT + (i & 1), 32 * ll1_stride, cnt,
+                             ep, v);
 #pragma unroll
         for (int u = 0; u < U; ++u)
           if (u < cnt) {
@@ -965,7 +971,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         yy = warp_sum(yy);
         if (b.has_vstar) yd = warp_sum(yd);
         if (lane == 0) {
-          uint4* out = b.pk_y + (size_t)q * blk + own_n + 3 * warp;
+          uint4* out = b.pk_y + (size_t)q * blk + own_n + 3 * (kShareWarps * (i & 1) + warp);
           packet_store(out, xy, ep);
           packet_store(out + 1, yy, ep);
           if (b.has_vstar) packet_store(out + 2, yd, ep);
@@ -1026,7 +1032,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         for (int r = t; r < nrec && ok; r += T) {
           uint4 v[1];
           const int w = r >= G ? 1 : 0;
-          ok = packets_wait<1, true>(p + (r - w * G) * blk + 3 * w, 0, 1, ep, v);
+          ok = packets_wait<1, true>(p + (r - w * G) * blk + 3 * (kShareWarps * (i & 1) + w), 0, 1,
+                                     ep, v);
           d += __hiloint2double((int)v[0].y, (int)v[0].x);
         }
         return d;

@@ -61,6 +61,29 @@ def test_step_kernel_shapes(m, n, c, dtype, method, kw):
     ctx.close()
 
 
+@pytest.mark.parametrize("m,n,c,dtype", [(8, 300, 33, "bf16"), (4, 400, 20, "f32"),
+                                         (1024, 700, 90, "f32"), (3000, 900, 120, "bf16")])
+def test_ctas_without_packets_over_many_calls(m, n, c, dtype):
+    """CTAs that own no packet of y run ahead of the others; over many calls of every kind of step no
+    packet is overwritten before a slower CTA has read it (the wait for it would run out and the
+    call report it), and the results stay bitwise the same."""
+    from eigenvaluecomputation_by_amm_b200 import AMMContext, column_major
+    A = torch.from_numpy(scaled_gaussian(m, n, seed=m, shift=0.05)).cuda()
+    A = A.to(torch.bfloat16) if dtype == "bf16" else A
+    ctx = AMMContext(m, n, c=c, step=24, dtype=dtype, vr_period=4)
+    ctx.set_matrix(column_major(A))
+    st = torch.from_numpy(states(c, 3).view(np.int32)).cuda()
+    x0 = torch.from_numpy(np.random.default_rng(4).standard_normal(m).astype(np.float32)).cuda()
+    want = {}
+    for call in range(60):
+        method = ("exact", "previous", "proposed")[call % 3]
+        ctx.set_rng_state(st)
+        ctx.power_method(method, x0)
+        eigs = ctx.trace()["eigs"]
+        assert np.array_equal(eigs, want.setdefault(method, eigs))
+    ctx.close()
+
+
 @pytest.mark.parametrize("step", [40, 1700])
 def test_trace_region_of_any_length(step):
     """A trace short enough for one copy and one that is copied piece by piece (1700 steps, stopped
