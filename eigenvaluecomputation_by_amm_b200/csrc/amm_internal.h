@@ -90,7 +90,7 @@ struct Buffers {
   double* vstar;       // may be null
   int32_t has_vstar;
   // sampling
-  uint32_t* states[2];   // xorshift states (c used); states[0]: committed at the call start
+  uint32_t* states;      // xorshift states (c used), as committed at the call start
   uint32_t* count[kListWindow];    // per slot: per-column multiplicity of the picks (n)
   uint32_t* chunk[kListWindow];    // per slot: distinct columns per chunk (nchunks)
   uint32_t* samples[kListWindow];  // per slot: raw picks in draw order (c)
@@ -179,8 +179,15 @@ cudaError_t launch_setup_panel(const Buffers& b, const PanelGeom& g, cudaStream_
 cudaError_t launch_build_cdf(const Buffers& b, int which, int keep_cdf, int sanity, cudaStream_t s);
 // Start of a call: x0 into y[1], scale, initial state, first picks.
 // no_normalize: use x0 as x_0 unscaled (single-product entry points).
+// memo (single products only): the caller's memo pair (null: zero) goes to the context's in the same
+// pass, and x0 to x_keep; every pointer 16-byte aligned.
+struct InitMemo {
+  const float* x_memo;
+  const float* y_memo;
+  float* x_keep;
+};
 cudaError_t launch_init(const Buffers& b, const CallCfg& cc, const float* x0, int no_normalize,
-                        cudaStream_t s);
+                        cudaStream_t s, const InitMemo* memo = nullptr);
 // Refill of the work-list window ahead of step iter (iter % kListWindow == 0): draw the picks of
 // the lists not yet drawn among the next kListWindow AMM steps.
 cudaError_t launch_sample(const Buffers& b, const CallCfg& cc, int iter, cudaStream_t s);
@@ -193,10 +200,10 @@ cudaError_t launch_compact(const Buffers& b, const CallCfg& cc, int iter, cudaSt
 // step's state.
 cudaError_t launch_iter_panel(const Buffers& b, const PanelGeom& g, const CallCfg& cc, int iter,
                               int iter_end, cudaStream_t s);
-// x_final = scale * y_last into dst (length m); y_last into ydst (optional); commits the
-// sampling states to states[0] and clears any pending picks.
+// x_final = scale * y_last into dst (length m); y_last into ydst and ydst2 (optional); commits the
+// sampling states and clears any pending picks.
 cudaError_t launch_finalize(const Buffers& b, const CallCfg& cc, float* xdst, float* ydst,
-                            cudaStream_t s);
+                            cudaStream_t s, float* ydst2 = nullptr);
 // Standalone helpers.
 cudaError_t launch_normalize(float* x, int m, cudaStream_t s);
 // Device-to-device copy of n floats by a kernel (a memcpy when unaligned).

@@ -157,7 +157,7 @@ struct SampleArgs {
 };
 
 // List number st.drawn + blockIdx.y of the window ahead of step iter, drawn from the call-start
-// states states[0] into its slot, if the window reaches it (see window_end).  The lists of the
+// states into its slot, if the window reaches it (see window_end).  The lists of the
 // window are drawn by independent grid rows.
 template <typename F>
 __global__ void __launch_bounds__(256) sample_kernel(const __grid_constant__ SampleArgs a) {
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256) sample_kernel(const __grid_constant__ Sam
   const int slot = list % kListWindow;
   const int which = list_weighting(cc, list);
   load_coarse<F>(b, which, coarse_s);
-  draw_samples<F>(b, which, b.states[0], list, b.count[slot], b.chunk[slot], b.samples[slot],
+  draw_samples<F>(b, which, b.states, list, b.count[slot], b.chunk[slot], b.samples[slot],
                   blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, coarse_s);
 }
 
@@ -346,6 +346,8 @@ struct InitArgs {
   CallCfg cc;
   const float* x0;
   int no_normalize;
+  int with_memo;  // the memo pair comes from `memo` (single products)
+  InitMemo memo;
 };
 
 __global__ void __launch_bounds__(1024) init_kernel(const __grid_constant__ InitArgs a) {
@@ -362,13 +364,22 @@ __global__ void __launch_bounds__(1024) init_kernel(const __grid_constant__ Init
   // 345-355, called first by every powerMethod_by_*); the single-product entry points keep
   // the memo their caller supplied
   const bool clear_memo = !a.no_normalize;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
   for (int k0 = 4 * t; k0 < b.m; k0 += 4 * blockDim.x) {  // m % 4 == 0
     const float4 v = __ldg(reinterpret_cast<const float4*>(x0 + k0));
     *reinterpret_cast<float4*>(y1 + k0) = v;
     if (clear_memo) {
-      *reinterpret_cast<float4*>(b.x_memo + k0) = make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(b.y_memo + k0) = make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(b.x_memo + k0) = zero;
+      *reinterpret_cast<float4*>(b.y_memo + k0) = zero;
+    } else if (a.with_memo) {
+      const float* xs = a.memo.x_memo;
+      const float* ys = a.memo.y_memo;
+      *reinterpret_cast<float4*>(b.x_memo + k0) =
+          xs ? __ldg(reinterpret_cast<const float4*>(xs + k0)) : zero;
+      *reinterpret_cast<float4*>(b.y_memo + k0) =
+          ys ? __ldg(reinterpret_cast<const float4*>(ys + k0)) : zero;
+      *reinterpret_cast<float4*>(a.memo.x_keep + k0) = v;
     }
     ss = fma((double)v.x, (double)v.x, ss);
     ss = fma((double)v.y, (double)v.y, ss);
@@ -393,7 +404,7 @@ __global__ void __launch_bounds__(1024) init_kernel(const __grid_constant__ Init
     st.used = 0;
     st.drawn = 0;
     st.steps_run = 0;
-    st.memo_zero = clear_memo ? 1 : 0;
+    st.memo_zero = clear_memo || (a.with_memo && !a.memo.x_memo) ? 1 : 0;
     if (!(s > 0.0) || !isfinite(s)) {
       atomicOr(b.status, (uint32_t)kDevNonFinite);
       st.done = 1;
@@ -410,6 +421,7 @@ struct FinalArgs {
   CallCfg cc;
   float* xdst;
   float* ydst;
+  float* ydst2;
 };
 
 __global__ void __launch_bounds__(kFinalThreads) finalize_kernel(const __grid_constant__ FinalArgs a) {
@@ -424,14 +436,15 @@ __global__ void __launch_bounds__(kFinalThreads) finalize_kernel(const __grid_co
     const float yv = ylast[k];
     if (a.xdst) a.xdst[k] = __fmul_rn(st.scale, yv);
     if (a.ydst) a.ydst[k] = yv;
+    if (a.ydst2) a.ydst2[k] = yv;
   }
   if (a.cc.uses_amm && !a.cc.sanity && !a.cc.ext_list) {
     // commit: each state advanced once per AMM step that ran
     if (st.used > 0)
       for (int k = gt; k < b.c; k += gs) {
-        uint32_t y = b.states[0][k];
+        uint32_t y = b.states[k];
         for (int r = 0; r < st.used; ++r) y = xorshift32(y);
-        b.states[0][k] = y;
+        b.states[k] = y;
       }
     // pending (drawn ahead, never consumed) lists are dropped: their states are not committed
     for (int list = st.used; list < st.drawn; ++list) {
@@ -678,7 +691,7 @@ __global__ void __launch_bounds__(512) rayleigh_kernel(const float* x_in, float*
   for (int k = t; k < m; k += blockDim.x) x_out[k] = __fmul_rn(scale_s, y[k]);
 }
 
-// Draw c indices from states[0] without storing the advanced states.
+// Draw c indices from the states without storing the advanced states.
 template <typename F>
 __global__ void __launch_bounds__(256) sample_only_kernel(const __grid_constant__ Buffers b,
                                                           int which, uint32_t* idx) {
@@ -691,7 +704,7 @@ __global__ void __launch_bounds__(256) sample_only_kernel(const __grid_constant_
     cdf = reinterpret_cast<const F*>(b.cdf32[which]);
   const F total = cdf[b.n - 1];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < b.c; k += gridDim.x * blockDim.x) {
-    const float u = uniform_from(xorshift32(b.states[0][k]));
+    const float u = uniform_from(xorshift32(b.states[k]));
     F target;
     if constexpr (sizeof(F) == 8)
       target = __dmul_rn(total, static_cast<double>(u));
@@ -792,12 +805,14 @@ cudaError_t launch_gather_alpha(const Buffers& b, int64_t count, cudaStream_t s)
 }
 
 cudaError_t launch_init(const Buffers& b, const CallCfg& cc, const float* x0, int no_normalize,
-                        cudaStream_t s) {
+                        cudaStream_t s, const InitMemo* memo) {
   InitArgs a{};
   a.b = b;
   a.cc = cc;
   a.x0 = x0;
   a.no_normalize = no_normalize;
+  a.with_memo = memo ? 1 : 0;
+  if (memo) a.memo = *memo;
   return launch_pdl(init_kernel, dim3(1), dim3(1024), s, a);
 }
 
@@ -824,12 +839,13 @@ cudaError_t launch_compact(const Buffers& b, const CallCfg& cc, int iter, cudaSt
 }
 
 cudaError_t launch_finalize(const Buffers& b, const CallCfg& cc, float* xdst, float* ydst,
-                            cudaStream_t s) {
+                            cudaStream_t s, float* ydst2) {
   FinalArgs a{};
   a.b = b;
   a.cc = cc;
   a.xdst = xdst;
   a.ydst = ydst;
+  a.ydst2 = ydst2;
   int blocks = (b.m + kFinalThreads - 1) / kFinalThreads;
   if (blocks > 256) blocks = 256;
   return launch_pdl(finalize_kernel, dim3(blocks), dim3(kFinalThreads), s, a);

@@ -106,3 +106,42 @@ def test_trace_region_of_any_length(step):
     assert np.all(rel(tr["eigs"], ref.eigs[:k]) < RTOL_LAMBDA_F32)
     assert np.all(np.diff(tr["t_ns"]) > 0) and set(tr["distinct"]) == {n}
     ctx.close()
+
+
+@pytest.mark.parametrize("memo", ["none", "x", "both"])
+def test_single_product_aligned_and_misaligned_vectors(memo):
+    """A single product reads 16-byte aligned vectors in place and copies others first: the same
+    result, with and without a memo pair, and with y written over an input."""
+    import ctypes as C
+    from eigenvaluecomputation_by_amm_b200 import AMMContext, column_major
+    m, n, c = 260, 900, 80
+    A = torch.from_numpy(scaled_gaussian(m, n, seed=41, shift=0.1)).cuda()
+    st = torch.from_numpy(states(c, 42).view(np.int32)).cuda()
+    ctx = AMMContext(m, n, c=c)
+    ctx.set_matrix(column_major(A))
+    g = torch.Generator(device="cuda").manual_seed(43)
+    x, xm, ym = (torch.randn(m, device="cuda", generator=g) for _ in range(3))
+    xm = xm if memo != "none" else None
+    ym = ym if memo == "both" else None
+
+    def product(off, over_x):
+        def put(v):
+            if v is None:
+                return None
+            buf = torch.empty(m + 4, device="cuda")
+            buf[off:off + m] = v
+            return buf[off:off + m]
+        px, pxm, pym = put(x), put(xm), put(ym)
+        y = px if over_x else torch.empty(m, device="cuda")
+        ptr = lambda v: None if v is None else C.c_void_p(v.data_ptr())  # noqa: E731
+        ctx.set_rng_state(st)
+        rc = ctx.lib.amm_core_proposedAMM(ctx._ctx, ptr(px), ptr(pxm), ptr(pym), ptr(y), None, None)
+        torch.cuda.synchronize()
+        assert rc == 0
+        return y.clone()
+
+    want = product(0, False)
+    assert torch.isfinite(want).all() and float(want.abs().max()) > 0
+    for off, over_x in ((1, False), (0, True), (3, True)):
+        assert torch.equal(product(off, over_x), want)
+    ctx.close()
