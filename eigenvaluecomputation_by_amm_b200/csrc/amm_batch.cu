@@ -14,8 +14,10 @@
 // ring that keeps two or more groups in flight), forms the K·GC partial dots A_jᵀX over its
 // rows, reduces them across the team (warp butterfly, then shared memory for teams wider than a
 // warp) and accumulates Y += A_j·(A_jᵀX): the fused single-pass product of the main kernel.
-// Exact batches of 8 vectors take a tensor-core form of the same product instead (TF32
-// mma.sync with a hi + lo split, column tiles copied by TMA; see batch_kernel).
+// Where it pays (plan_gram) the exact products of blocks of 4 or 8 go through C = A·Aᵀ, formed once
+// per run on tcgen05 (amm_gram.cu), as C·X (cx_product).  Exact batches of 8 vectors take a
+// tensor-core form of the product through A otherwise (TF32 mma.sync with a hi + lo split, column
+// tiles copied by TMA; see batch_kernel).
 // After the pass the team partials of Y are summed in a fixed order, the Gram matrices
 // G = YᵀY and H = XᵀY are reduced in FP64, X <- Y·R⁻¹ (Cholesky QR), and every rr_period
 // iterations (and at the end) H is diagonalised by a warp-parallel cyclic Jacobi in FP64: its
@@ -2193,9 +2195,9 @@ static double direct_clocks(const Mat& x, const amm_batch_config& cfg) {
 // Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which forming C
 // (2500 clocks per 128 x 128 tile and 64 columns) and the products with it (m·m·nvec FMAs at 128 a
 // clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only with the tile shape
-// left to the library (a fixed one asks for its product) and an even block.  Returns C's floats
-// in all; `cost`: estimated clocks per matrix.
-static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg,
+// left to the library (a fixed one asks for its product) and an even block; none without `with_c`.
+// Returns C's floats in all; `cost`: estimated clocks per matrix.
+static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c,
                          std::vector<double>& cost) {
   const double p = exact_products(cfg);
   int64_t floats = 0;
@@ -2210,7 +2212,7 @@ static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg,
     const double form = t * (t + 1) / 2 * chunks * 2500.0;
     const double by_c = p * (double)x.m * (double)x.m * (double)cfg.nvec / 96.0;
     cost[i] = direct_clocks(x, cfg);
-    if (cfg.tile_gc == 0 && cfg.nvec % 2 == 0 && form + by_c < 0.8 * direct) {
+    if (with_c && cfg.tile_gc == 0 && cfg.nvec % 2 == 0 && form + by_c < 0.8 * direct) {
       x.C = reinterpret_cast<float*>(1);  // placed by place_gram
       floats += (int64_t)x.ldc * x.ldc;
       cost[i] += by_c - direct;  // (C is formed by a launch of its own)
@@ -2237,8 +2239,9 @@ static void place_gram(std::vector<Mat>& ms, float* mem, std::vector<amm::batch:
                    });
 }
 
-int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t count,
-                     const amm_batch_config* cfg, int device) {
+// with_c: matrices may be multiplied as C·X, with memory for C
+static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t count,
+                        const amm_batch_config* cfg, int device, bool with_c) {
   if (!out || !mats || !cfg || count < 1 || count > (1 << 20)) return AMM_ERR_INVALID_ARGUMENT;
   *out = nullptr;
   if (cfg->nvec != 1 && cfg->nvec != 4 && cfg->nvec != 8) return AMM_ERR_UNSUPPORTED;
@@ -2276,19 +2279,19 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
     cols += x.n;
   }
   std::vector<double> cost;
-  const int64_t c_floats = plan_gram(ms, *cfg, cost);
+  const int64_t c_floats = plan_gram(ms, *cfg, with_c, cost);
   amm_batch* b = new amm_batch();
   b->device = device;
   b->cfg = *cfg;
   b->count = count;
   Guard g(device);
-  // C of the matrices multiplied as C·X (an allocation of its own: without room for it every
-  // product reads A)
-  if (c_floats > 0 && cudaMalloc(&b->c_mem, sizeof(float) * (size_t)c_floats) != cudaSuccess) {
-    cudaGetLastError();
-    b->c_mem = nullptr;
-    for (Mat& x : ms) x.C = nullptr;
-    for (int64_t i = 0; i < count; ++i) cost[i] = direct_clocks(ms[i], *cfg);
+  if (c_floats > 0) {
+    const cudaError_t ce = cudaMalloc(&b->c_mem, sizeof(float) * (size_t)c_floats);
+    if (ce != cudaSuccess) {
+      cudaGetLastError();
+      delete b;
+      return ce == cudaErrorMemoryAllocation ? AMM_ERR_OUT_OF_MEMORY : fail(ce, "cudaMalloc");
+    }
   }
   std::vector<amm::batch::GramTile> tiles;
   if (b->c_mem) place_gram(ms, b->c_mem, tiles);
@@ -2331,6 +2334,7 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   const size_t o_tmaps = with_tmaps ? carve(sizeof(CUtensorMap) * count, 256) : 0;
   cudaError_t e = cudaMalloc(&b->mem, bytes);
   if (e != cudaSuccess) {
+    cudaGetLastError();
     if (b->c_mem) cudaFree(b->c_mem);
     delete b;
     return e == cudaErrorMemoryAllocation ? AMM_ERR_OUT_OF_MEMORY : fail(e, "cudaMalloc");
@@ -2384,6 +2388,13 @@ int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t coun
   }
   *out = b;
   return AMM_OK;
+}
+
+int amm_batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t count,
+                     const amm_batch_config* cfg, int device) {
+  const int rc = batch_create(out, mats, count, cfg, device, true);
+  // without room for C every product reads A
+  return rc == AMM_ERR_OUT_OF_MEMORY ? batch_create(out, mats, count, cfg, device, false) : rc;
 }
 
 int amm_batch_destroy(amm_batch* b) {

@@ -85,3 +85,13 @@ def test_variance_reduced_products_by_c(amm_lib, cluster):
     assert float(((a.lam[:, 0] - b.lam[:, 0]).abs() / b.lam[:, 0]).max()) < 2e-6
     a.close()
     b.close()
+
+
+def test_without_room_for_c_the_products_read_a():
+    """C of all the matrices (206 GB) does not fit the device: the solver is made without it."""
+    from eigenvaluecomputation_by_amm_b200 import BatchSolver
+    A = torch.zeros(4096, 2048, device="cuda").t()
+    free0 = torch.cuda.mem_get_info()[0]
+    solver = BatchSolver([A] * 12288, nvec=8, max_iter=20, tol=0.0)
+    assert free0 - torch.cuda.mem_get_info()[0] < 4 << 30
+    solver.close()
