@@ -779,7 +779,7 @@ def run_ours(args, rank, world):
         "c5_grad_64x512x2048": c5,
         "roofline": {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm,
                      "traffic": traffic, "peak_source": src,
-                     "kernel": f"panel_kernel<bf16> persistent step kernel inside the timed "
+                     "kernel": f"step_kernel<bf16> persistent step kernel inside the timed "
                                f"solves: steps 1..{amm_steps - 1} of each of the {len(step_clocks)} "
                                f"solves ({ins_steps['exact']} exact + {ins_steps['amm']} proposed "
                                "AMM steps), timed by the kernel's own device clock stamp at the "

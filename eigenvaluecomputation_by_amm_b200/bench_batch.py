@@ -158,7 +158,9 @@ def batch_report(count=512, iters=20, check=32, modes=("exact", "amm", "amm_vr")
         if mode == "exact":
             ach = bytes_per_product * iters / (t_one * 1e-3) / 1e9
             res["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
-                               "frac": ach / hbm, "peak_source": src}
+                               "frac": ach / hbm, "peak_source": src,
+                               "note": "one read of A per product counted; matrices multiplied "
+                                       "through C = A·Aᵀ read A once per run"}
             t_each = time_runs(bs, each=True)
             res["one_cta_launch_per_matrix_matrices_per_s"] = count * 1000.0 / t_each
         out[mode] = res

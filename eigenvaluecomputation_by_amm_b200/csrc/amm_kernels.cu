@@ -4,8 +4,9 @@
 //   init_kernel      x0, the memo pair, the first state
 //   sample_kernel,   every kListWindow steps: the picks (xorshift32 + inverse CDF) of the next
 //   compact_kernel   kListWindow AMM steps and their sorted distinct work lists
-//   panel_kernel     one launch per step (amm_panel.cu): the product over the step's columns,
-//                    the grid-wide reduction into y and the Rayleigh quotient / next state
+//   step_kernel      one launch per window (amm_step.cu; panel_kernel of amm_panel.cu with clusters
+//                    or too few SMs): per step the product over its columns, the grid-wide
+//                    reduction into y and the Rayleigh quotient / next state
 //   finalize_kernel  x_final, y_final, the committed sampling states
 // plus the CDF construction of the set-up and the standalone helpers.
 #include <cuda_bf16.h>

@@ -2,8 +2,10 @@
 //
 //   y_part = Σ_{k in this CTA's columns} coef_k · A_k,   coef_k = f(A_kᵀ·dx)
 //
-// for one power-method step (all n columns for an exact step, the distinct sampled columns for
-// an AMM step) and for the set-up pass (coef_j = α_j, plus FP64 column statistics).
+// for the set-up pass (coef_j = α_j, plus FP64 column statistics), and for the power-method steps (all
+// n columns for an exact step, the distinct sampled columns for an AMM step) where the packet
+// exchange of amm_step.cu does not apply: thread-block clusters, or a device or MIG slice with too few
+// SMs for it.
 //
 // One persistent CTA per SM owns a contiguous range of the column list and all m rows.  Thread 0
 // streams the columns, GC per group, into a ring of NS shared-memory stages with 1-D TMA bulk
