@@ -17,10 +17,15 @@
 // long for N = 128 as for N = 256 (128 x 128 tiles: 6.7 ms for the 476 matrices of the 512-matrix
 // batch that are multiplied as C·X).  Per chunk every thread converts 2 + 4 float4 (4 consecutive
 // rows of a column: one coalesced 16-byte load, three 8-byte stores into the 128-byte-swizzled
-// MN-major planes), one thread issues the 12 products, and while they run the threads load the next
-// chunk and add the one before from tensor memory (two accumulators, two stages of planes).
-// What bounds it: the products, about 150 clocks each, and shared-memory bandwidth (per chunk
-// 72 KB of planes written, 144 KB read, at 128 bytes a clock).
+// MN-major planes), one thread issues the 12 products, and while they run the threads add the chunk before from
+// tensor memory (two accumulators, two stages of planes).  The next chunk's loads are issued before
+// the barrier, so that their latency passes while the warps meet.
+// What bounds it: the converting threads (64 accumulators and 24 loaded values of 128 registers
+// each), then the products, about 150 clocks each, and shared-memory bandwidth (per chunk 72 KB of
+// planes written, 144 KB read, at 128 bytes a clock).  The whole run of the 512-matrix batch: loads
+// after the barrier, 16 tensor-memory columns at a time 14.3 ms; loads before it 14.2; 8 columns at a
+// time (fewer spills) 13.2, with the loads after the barrier 13.9; 32-bit shared-memory addresses and
+// one column pointer 12.8.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -73,19 +78,20 @@ __device__ __forceinline__ void tmem_fence_before() {
 __device__ __forceinline__ void tmem_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-// 16 columns of this warp's 32 tensor-memory lanes, added to acc
-__device__ __forceinline__ void tmem_add16(uint32_t addr, float* acc) {
-  uint32_t r[16];
+__device__ __forceinline__ void st_shared(uint32_t addr, uint32_t x, uint32_t y) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(addr), "r"(x), "r"(y) : "memory");
+}
+// 8 columns of this warp's 32 tensor-memory lanes, added to acc
+__device__ __forceinline__ void tmem_add8(uint32_t addr, float* acc) {
+  uint32_t r[8];
   asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-        "=r"(r[14]), "=r"(r[15])
+        "=r"(r[7])
       : "r"(addr));
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < 16; ++i) acc[i] += __uint_as_float(r[i]);
+  for (int i = 0; i < 8; ++i) acc[i] += __uint_as_float(r[i]);
 }
 
 // two floats to BF16 (nearest), x in the low half
@@ -108,10 +114,12 @@ __global__ void __launch_bounds__(kGramThreads, 1)
     gram_kernel(const Mat* __restrict__ mats, const GramTile* __restrict__ tiles, int ntiles,
                 uint32_t* queue) {
   extern __shared__ __align__(16) unsigned char gram_smem[];
-  unsigned char* planes = gram_smem + ((1024u - (smem_addr(gram_smem) & 1023u)) & 1023u);
+  const uint32_t planes = (smem_addr(gram_smem) + 1023u) & ~1023u;
   __shared__ uint64_t bar[2];     // products of a stage done
   __shared__ uint32_t tmem_s;
   __shared__ int tile_s;
+  // of the products: the instruction; the column operand's first byte, rows and bytes per plane
+  __shared__ uint32_t op_s[4];
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -129,7 +137,7 @@ __global__ void __launch_bounds__(kGramThreads, 1)
   __syncthreads();
   tmem_fence_after();
   const uint32_t tmem = tmem_s;
-  uint32_t ph[2] = {0u, 0u};  // phase parity of the two stages (alike in every thread)
+  uint32_t ph = 0u;           // phase parity of the two stages, a bit each (alike in every thread)
   bool dead = false;          // a wait gave up: no more products, every tile is NaN
   // this thread's part of an accumulator: lane quarter warp % 4, columns 64·(warp / 4) ..
   const int seg = 64 * (warp >> 2);
@@ -150,39 +158,47 @@ __global__ void __launch_bounds__(kGramThreads, 1)
     // an even row block's last tile is its diagonal block alone: the rows serve as both operands
     const bool diag = 2 * tl.tj == tl.ti;
     const int ncol = diag ? kRows : min(kCols, (M.ldc - kCols * tl.tj + 15) & ~15);
-    const uint32_t instr = kInstr | ((uint32_t)(ncol >> 3) << 17);
+    // (what only the issuing thread or the tile's end needs is kept out of the registers)
+    if (t == 0) {
+      op_s[0] = kInstr | ((uint32_t)(ncol >> 3) << 17);
+      op_s[1] = diag ? 0u : 3u * kPlaneA;
+      op_s[2] = diag ? kRows : kCols;
+      op_s[3] = diag ? kPlaneA : kPlaneB;
+    }
     const int nchunk = (n + kChunk - 1) / kChunk;
     const int ra0 = kRows * tl.ti + 4 * lane, rb0 = kCols * tl.tj + 4 * lane;
-    // rows r0 .. r0 + 3 of column k (zeros outside the matrix)
-    auto load4 = [&](int r0, int k) -> float4 {
+    // rows r0 .. r0 + 3 of a column at p (zeros outside the matrix; left: rows from r0 to the end)
+    auto load4 = [](const float* p, int left) -> float4 {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (k < n && r0 < m) {
-        const float* p = M.A + (int64_t)k * M.ld + r0;
-        if (r0 + 4 <= m) {
-          v = __ldg(reinterpret_cast<const float4*>(p));
-        } else {  // the last rows: nothing past row m is read
-          v.x = __ldg(p);
-          if (r0 + 1 < m) v.y = __ldg(p + 1);
-          if (r0 + 2 < m) v.z = __ldg(p + 2);
-        }
+      if (left >= 4) {
+        v = __ldg(reinterpret_cast<const float4*>(p));
+      } else if (left > 0) {  // the last rows: nothing past row m is read
+        v.x = __ldg(p);
+        if (left > 1) v.y = __ldg(p + 1);
+        if (left > 2) v.z = __ldg(p + 2);
       }
       return v;
     };
+    // this thread's rows of the chunk's first column of its two
+    const float* pa = M.A + (int64_t)(2 * warp) * M.ld + ra0;
+    const int ab = rb0 - ra0;  // (from the row operand's rows to the column operand's)
+    const int64_t ld = M.ld;
+    const int la = m - ra0, lb = diag ? 0 : m - rb0;
+    int left_k = n - 2 * warp;  // columns from this thread's first one to the end
     float4 ra[2], rb[2][2];  // [column], [128 rows][column]
-    auto load_chunk = [&](int kc) {
-      const int k0 = kc * kChunk + 2 * warp;
+    auto load_chunk = [&]() {  // the chunks in turn
 #pragma unroll
-      for (int j = 0; j < 2; ++j) ra[j] = load4(ra0, k0 + j);
-      if (!diag) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          if (128 * h < ncol)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) rb[h][j] = load4(rb0 + 128 * h, k0 + j);
+      for (int j = 0; j < 2; ++j) {
+        const bool in = j < left_k;
+        ra[j] = load4(pa + j * ld, in ? la : 0);
+        rb[0][j] = load4(pa + ab + j * ld, in ? lb : 0);
+        rb[1][j] = load4(pa + ab + j * ld + 128, in ? lb - 128 : 0);
       }
+      pa += kChunk * ld;
+      left_k -= kChunk;
     };
     // 128 rows of an operand of `rows` rows, from its row block `blk` (of 64) on
-    auto convert = [&](const float4 (&r)[2], unsigned char* base, uint32_t rows, uint32_t blk,
+    auto convert = [&](const float4 (&r)[2], uint32_t base, uint32_t rows, uint32_t blk,
                        uint32_t plane) {
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
@@ -194,7 +210,7 @@ __global__ void __launch_bounds__(kGramThreads, 1)
                              ((piece ^ c) << 4) + half * 8u;
 #pragma unroll
         for (int p = 0; p < 3; ++p)
-          *reinterpret_cast<uint2*>(base + p * plane + off) = make_uint2(lo[p], hi[p]);
+          st_shared(base + p * plane + off, lo[p], hi[p]);
       }
     };
     float acc[64];
@@ -203,37 +219,36 @@ __global__ void __launch_bounds__(kGramThreads, 1)
     // add chunk kc's accumulator once its products are done
     auto promote = [&](int kc) {
       const int s = kc & 1;
-      if (!dead && !mbar_wait_bounded(&bar[s], ph[s])) dead = true;
-      ph[s] ^= 1u;
+      if (!dead && !mbar_wait_bounded(&bar[s], (ph >> s) & 1u)) dead = true;
+      ph ^= 1u << s;
       tmem_fence_after();
       __syncwarp();
       if (seg < ncol) {  // warp-uniform
 #pragma unroll
-        for (int h = 0; h < 4; ++h)
-          tmem_add16(acc_addr + (uint32_t)(s * kCols + 16 * h), acc + 16 * h);
+        for (int h = 0; h < 8; ++h)
+          tmem_add8(acc_addr + (uint32_t)(s * kCols + 8 * h), acc + 8 * h);
       }
       tmem_fence_before();
     };
-    // row r, columns c0 .. c0 + 63 of C; what lies in the tile but past ldc is left out
-    const int r = kRows * tl.ti + 32 * (warp & 3) + lane, c0 = kCols * tl.tj + seg;
-    const bool live = r < M.ldc && seg < ncol;
-    load_chunk(0);
+    load_chunk();
 #pragma unroll 1
     for (int kc = 0; kc < nchunk; ++kc) {
       const int s = kc & 1;
-      unsigned char* st = planes + s * kStage;
+      const uint32_t st = planes + (uint32_t)(s * kStage);
       convert(ra, st, kRows, 0, kPlaneA);  // (the stage's last products were waited for)
       if (!diag) {
         convert(rb[0], st + 3 * kPlaneA, kCols, 0, kPlaneB);
         if (ncol > 128) convert(rb[1], st + 3 * kPlaneA, kCols, 2, kPlaneB);
       }
       fence_proxy_async_smem();
+      if (kc + 1 < nchunk) load_chunk();
       dead = __syncthreads_or(dead ? 1 : 0) != 0;
       if (t == 0 && !dead) {
         tmem_fence_after();
-        const uint32_t d = tmem + (uint32_t)(s * kCols);
-        const uint32_t a0 = smem_addr(st), b0 = diag ? a0 : a0 + 3 * kPlaneA;
-        const uint32_t brows = diag ? kRows : kCols, bplane = diag ? kPlaneA : kPlaneB;
+        const uint32_t d = *const_cast<volatile uint32_t*>(&tmem_s) + (uint32_t)(s * kCols);
+        const volatile uint32_t* op = op_s;
+        const uint32_t instr = op[0], a0 = st, b0 = a0 + op[1];
+        const uint32_t brows = op[2], bplane = op[3];
         // (plane of A, plane of B), the small products first
         constexpr int pa[6] = {1, 0, 2, 0, 1, 0}, pb[6] = {1, 2, 0, 1, 0, 0};
         bool add = false;
@@ -247,7 +262,6 @@ __global__ void __launch_bounds__(kGramThreads, 1)
           }
         mma_commit(&bar[s]);
       }
-      if (kc + 1 < nchunk) load_chunk(kc + 1);
       if (kc > 0) promote(kc - 1);
     }
     promote(nchunk - 1);
@@ -256,17 +270,22 @@ __global__ void __launch_bounds__(kGramThreads, 1)
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = __int_as_float(0x7fffffff);
     }
-    // the tile, and its mirror image unless it is in the diagonal block (rows and columns of [m, ldc)
-    // are zeros, computed from zero rows)
-    if (live) {
+    // row r, columns c0 .. c0 + 63 of C (what lies in the tile but past ldc is left out), and their
+    // mirror image unless in the diagonal block (rows and columns of [m, ldc) are zeros, computed from
+    // zero rows)
+    const GramTile te = tiles[*const_cast<volatile int*>(&tile_s)];
+    float* const C = mats[te.mat].C;
+    const int ldc = mats[te.mat].ldc;
+    const int r = kRows * te.ti + 32 * (warp & 3) + lane, c0 = kCols * te.tj + seg;
+    if (r < ldc && seg < ncol) {
 #pragma unroll
       for (int i = 0; i < 64; ++i)
-        if (c0 + i < M.ldc) M.C[(int64_t)(c0 + i) * M.ldc + r] = acc[i];
-      if (c0 / kRows != tl.ti) {
+        if (c0 + i < ldc) C[(int64_t)(c0 + i) * ldc + r] = acc[i];
+      if (c0 / kRows != te.ti) {
 #pragma unroll
         for (int i = 0; i < 64; i += 4)
-          if (c0 + i < M.ldc)
-            *reinterpret_cast<float4*>(M.C + (int64_t)r * M.ldc + c0 + i) =
+          if (c0 + i < ldc)
+            *reinterpret_cast<float4*>(C + (int64_t)r * ldc + c0 + i) =
                 make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
       }
     }
