@@ -29,10 +29,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <tuple>
 #include <cstdint>
 #include <cstring>
+#include <functional>
 #include <map>
+#include <queue>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "amm.h"
@@ -182,29 +185,39 @@ __device__ __forceinline__ void rr_pair(int K, int r, int s, int* p, int* q) {
   *q = a < b ? b : a;
 }
 
-// 1/sqrt(x) to FP64 rounding for x in FP32's normal range: two of Newton's steps from the FP32
-// reciprocal square root, without a branch (so that two of them interleave)
-__device__ __forceinline__ double rsqrt_newton(double x) {
-  double y = (double)rsqrtf((float)x);
-  const double hx = 0.5 * x;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) y *= fma(-(hx * y), y, 1.5);
-  return y;
-}
-
-// The rotation (c, s) that annihilates h_pq: d = h_qq − h_pp, b = 2·h_pq, cos 2θ = |d|/h, sin 2θ =
-// sign(d)·b/h, h = sqrt(d² + b²); entries scaled to at most about 1 (below 1e-18 of that there is
-// nothing to rotate).
+// The rotation (c, s) that annihilates h_pq: t = tan θ = sign(d)·b / (|d| + sqrt(d² + b²)), d = h_qq −
+// h_pp, b = 2·h_pq, to FP32 accuracy from d and b scaled by an exact power of two (max(|d|, |b|) in
+// [1, 2)); (c, s) = (1, t)/sqrt(1 + t²) in FP32, then two Newton steps x <- x·(3 − (c² + s²))/2 in FP64
+// make the rotation orthogonal to FP64 rounding.  An angle off by FP32 rounding leaves h_pq at ~1e-7
+// of its size instead of 0, which the next sweep removes; the eigenvalues depend only on the
+// orthogonality.
 __device__ __forceinline__ void jacobi_angle(double hpp, double hqq, double hpq, double* c,
                                              double* s) {
-  const double d = hqq - hpp, b = hpq + hpq;
-  const double h2 = fma(d, d, b * b);
-  const double rh = rsqrt_newton(h2);
-  const double c2 = fma(0.5 * fabs(d), rh, 0.5);  // cos²θ, in [1/2, 1]
-  const double rc = rsqrt_newton(c2);
-  const bool rot = hpq != 0.0 && h2 > 1e-36;
-  *c = rot ? c2 * rc : 1.0;
-  *s = rot ? copysign(0.5, d) * (b * rh) * rc : 0.0;
+  const double dd = hqq - hpp, bb = 2.0 * hpq;
+  const double mx = fmax(fabs(dd), fabs(bb));
+  const int ex = (int)((__double_as_longlong(mx) >> 52) & 0x7ff);
+  const double sc = __longlong_as_double((long long)(2046 - min(ex, 2045)) << 52);
+  const float df = (float)(dd * sc), bf = (float)(bb * sc);
+  const float tf = copysignf(1.f, df) * __fdividef(bf, fabsf(df) + sqrtf(fmaf(df, df, bf * bf)));
+  const float cf = rsqrtf(fmaf(tf, tf, 1.f));
+  double cc = (double)cf, ss = (double)(tf * cf);
+#pragma unroll
+  for (int nw = 0; nw < 2; ++nw) {
+    const double f = fma(-0.5, fma(cc, cc, ss * ss), 1.5);
+    cc *= f;
+    ss *= f;
+  }
+  *c = hpq != 0.0 ? cc : 1.0;
+  *s = hpq != 0.0 ? ss : 0.0;
+}
+
+// (a, b)·[c s; -s c], the rounding of each term stated: left to the compiler it would follow the code
+// around it, and the blocks that sampled batches rotate can be singular to FP32 (see sampled_cluster)
+__device__ __forceinline__ double rot_first(double c, double s, double a, double b) {
+  return __fma_rn(c, a, -__dmul_rn(s, b));
+}
+__device__ __forceinline__ double rot_second(double c, double s, double a, double b) {
+  return __fma_rn(s, a, __dmul_rn(c, b));
 }
 
 // Cyclic Jacobi on the symmetric K x K matrix H (FP64, shared memory) by one warp; V receives
@@ -221,17 +234,6 @@ __device__ void jacobi_warp(double* H, double* V, int lane) {
   for (int i = lane; i < K * K; i += 32) V[i] = (i / K == i % K) ? 1.0 : 0.0;
   __syncwarp();
   if constexpr (K > 1) {
-    // H scaled by the power of two that brings its largest diagonal entry to [1, 2)
-    double mx = 0.0;
-#pragma unroll
-    for (int i = 0; i < K; ++i) mx = fmax(mx, fabs(H[i * K + i]));
-    const int ex = (int)((__double_as_longlong(mx) >> 52) & 0x7ff);
-    const bool scaled = ex > 0 && ex < 2046;  // neither zero nor infinite or NaN
-    const double up = scaled ? __longlong_as_double((long long)(2046 - ex) << 52) : 1.0;
-    const double down = scaled ? __longlong_as_double((long long)ex << 52) : 1.0;
-    __syncwarp();
-    for (int i = lane; i < K * K; i += 32) H[i] *= up;
-    __syncwarp();
     constexpr int NPR = K / 2;                      // pairs of a round
     constexpr int NH = NPR * NPR, NVL = K * NPR / 2;  // lanes on H and on V
     const bool on_h = lane < NH, act = lane < NH + NVL;
@@ -287,19 +289,17 @@ __device__ void jacobi_warp(double* H, double* V, int lane) {
         // pair b.  Selects, no branch: lanes that part here stay parted for the rounds that follow
         const double c0 = on_h ? cb : ca, s0 = on_h ? snb : sna;
         const double cr = on_h ? ca : 1.0, sr = on_h ? sna : 0.0;
-        const double t00 = c0 * e00 - s0 * e01, t01 = s0 * e00 + c0 * e01;
-        const double t10 = cb * e10 - snb * e11, t11 = snb * e10 + cb * e11;
+        const double t00 = rot_first(c0, s0, e00, e01), t01 = rot_second(c0, s0, e00, e01);
+        const double t10 = rot_first(cb, snb, e10, e11), t11 = rot_second(cb, snb, e10, e11);
         if (act) {
-          B[i00] = cr * t00 - sr * t10;
-          B[i01] = cr * t01 - sr * t11;
-          B[i10] = sr * t00 + cr * t10;
-          B[i11] = sr * t01 + cr * t11;
+          B[i00] = rot_first(cr, sr, t00, t10);
+          B[i01] = rot_first(cr, sr, t01, t11);
+          B[i10] = rot_second(cr, sr, t00, t10);
+          B[i11] = rot_second(cr, sr, t01, t11);
         }
         __syncwarp();
       }
     }
-    if (lane < K) H[lane * K + lane] *= down;  // (the diagonal is what is read)
-    __syncwarp();
   }
 }
 
@@ -540,8 +540,9 @@ __device__ __noinline__ void ritz_step(const Args& a, int mi, int it, double* Gm
 // S = X_memoᵀ·X (FP64 sums over team 0's rows, into Svr) and D = X − X_memo·S in place of X
 // (X saved to Xsave, restored by vr_add_memo after the product); called by every thread of the CTA.
 // The memo slots hold a thread's 4 rows as K float4s, float4 i of thread t at i·kThreads + t: every
-// access is coalesced, and every thread reads back only what it wrote.  For 8 vectors S is formed
-// on the FP64 tensor cores from a copy of X_memo in shared memory (`Ys`), as the Gram matrices are.
+// access is coalesced, and every thread reads back only what it wrote.  The sums of S: over a
+// thread's 4 rows in turn, then a butterfly over the warp (K entries of S at a time), then over team 0's
+// warps in turn.
 template <int K>
 __device__ __forceinline__ void memo_load(const float* p, int t, float (&v)[4][K]) {
 #pragma unroll
@@ -560,42 +561,27 @@ __device__ __forceinline__ void memo_store(float* p, int t, const float (&v)[4][
         make_float4(v[4 * i / K][4 * i % K], v[(4 * i + 1) / K][(4 * i + 1) % K],
                     v[(4 * i + 2) / K][(4 * i + 2) % K], v[(4 * i + 3) / K][(4 * i + 3) % K]);
 }
-__device__ __forceinline__ void mma_f64(double (&d)[2], double a, double b);
-
 template <int K>
-__device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xsave, float* Ys,
-                                           double* gpart, float* Svr, int P, int r0, int t,
-                                           int warp, int lane, int team) {
+__device__ __noinline__ void vr_difference(const float* Xm, float* Xs, float* Xsave, double* gpart,
+                                           float* Svr, int P, int r0, int t, int warp, int lane,
+                                           int team) {
   const int tw = P / 32;  // warps of team 0
   float xm[4][K];
-  if (team == 0) memo_load<K>(Xm, t, xm);
-  if constexpr (K == 8) {
-    if (team == 0) {  // warp-uniform
-      y_store<K>(Ys, t, xm);
-      __syncwarp();
-      double d[2] = {0.0, 0.0};
-      const int g = lane >> 2, tq = lane & 3, rb = 128 * warp;
-#pragma unroll 4
-      for (int k = 0; k < 32; ++k) {
-        const int row = rb + 4 * k + tq;
-        mma_f64(d, (double)Ys[yat<K>(row, g)], (double)Xs[xs_idx<K>(g, row)]);
-      }
-      gpart[warp * K * K + g * K + 2 * tq] = d[0];
-      gpart[warp * K * K + g * K + 2 * tq + 1] = d[1];
-    }
-  } else if (warp < tw) {
-    for (int ab = 0; ab < K * K; ++ab) {
-      const int va = ab / K, vb = ab % K;
-      double sv = 0.0;
+  if (team == 0) {  // warp-uniform
+    memo_load<K>(Xm, t, xm);
+#pragma unroll 1
+    for (int vb = 0; vb < K; ++vb) {
+      double x[4], d[K];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float x = 0.f;
+      for (int e = 0; e < 4; ++e) x[e] = (double)Xs[xs_idx<K>(vb, r0 + e)];
 #pragma unroll
-        for (int v = 0; v < K; ++v) x = v == va ? xm[e][v] : x;
-        sv = fma((double)x, (double)Xs[xs_idx<K>(vb, r0 + e)], sv);
+      for (int va = 0; va < K; ++va) {
+        d[va] = 0.0;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) d[va] = fma((double)xm[e][va], x[e], d[va]);
       }
-      sv = warp_sum(sv);
-      if (lane == 0) gpart[warp * K * K + ab] = sv;
+      const double r = warp_reduce_multi<double, K>(d, lane);  // value lane / (32 / K)
+      if (lane % (32 / K) == 0) gpart[warp * K * K + lane / (32 / K) * K + vb] = r;
     }
   }
   __syncthreads();
@@ -1253,12 +1239,12 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // the sampled product multiplies, D = X − X_memo·S, in place of X; Y_memo·S is added,
       // and X put back, once the product is summed ----
       const bool use_d = wamm && memo;
-      if (use_d) vr_difference<K>(Xm, Xs, Xsave, yred, gpart, Svr, P, r0, t, warp, lane, team);
+      if (use_d) vr_difference<K>(Xm, Xs, Xsave, gpart, Svr, P, r0, t, warp, lane, team);
       const float* Xsrc = Xs;  // X, or D in its place
       // ---- Y = C·X (or its AMM estimate): the fused pass over the columns (team-local) ----
       const bool rows = r0 < m;
       int buf = 0;
-      const bool by_c = K % 2 == 0 && M.C != nullptr && !wamm;  // an exact product as C·X
+      const bool by_c = K % 2 == 0 && M.C != nullptr;  // the product as C·X (exact batches)
       if (by_c) {
         // (nothing that this kernel keeps in registers is passed to an out-of-line function by
         // address: it would live in local memory, and the L1 left beside the shared memory is
@@ -1772,7 +1758,8 @@ struct amm_batch {
   float* c_mem = nullptr;
   amm::batch::GramTile* d_tiles = nullptr;
   int ntiles = 0;
-  std::vector<double> cost;  // estimated clocks of a run per matrix, for the order and the plan
+  std::vector<double> cost;  // estimated clocks of a run per matrix, for the order and the plan (sampled
+                             // batches: m·n)
   // device memory (one allocation)
   void* mem = nullptr;
   Mat* d_mats = nullptr;
@@ -1973,6 +1960,74 @@ int launch_run(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cuda
                 (int)b->cfg.max_iter, b->d_order, (int)b->count, s);
 }
 
+// Exact products of `it` products of a sampled run with variance reduction.
+int64_t exact_of_sampled(const amm_batch_config& cfg, int64_t it) {
+  return cfg.vr_period > 0 ? it / cfg.vr_period + (it % cfg.vr_period != 0 ? 1 : 0) : 0;
+}
+
+// CTAs per matrix of a sampled batch of blocks (4 columns per group), from the sizes alone.
+//
+// A product sampled before the first memo has the rank of its distinct picks.  Where few columns carry
+// a matrix's weight they are fewer than the block's vectors, and the block's last vectors are rounding:
+// the order of the sums, which the cluster size and the group size set, shows in the Ritz values that
+// follow (1e-3 of them over 111 matrices of 8 to 80 picks).  A tiling taken by the clock would make
+// results follow the clock.  So the time of a run is estimated per cluster size, with the
+// matrices handed to the clusters in order, each to the first that is free, and the smallest is taken:
+// us per matrix and product, fixed part by team width (32 .. 512 threads), column groups, and what a
+// cluster adds.  Fitted to the times of every cluster size over 502 batches of 8 to 600 matrices (m
+// 16-2048, n 64-8192, c = n/4 .. n/32): the fastest size in 92 % of them, 0.5 % slower on average.
+// (Times of the kernel while its tilings were still timed, 22.9 ms for the 512-matrix batch: other
+// constants would give such batches other results.)
+struct SampledCost {
+  double fixed[5], group[5];   // by log2(threads of a team / 32)
+  double draw, join, join_row; // a sampled product; a cluster's sums, per CTA and team width
+  double distinct;             // distinct columns per pick
+};
+constexpr SampledCost kSampled4 = {{18.5, 18.3, 17.7, 21.6, 24.3}, {1.31, 1.60, 1.60, 1.68, 1.75},
+                                   2.1, 4.6, 0.312, 0.3};
+constexpr SampledCost kSampled8 = {{45.4, 50.0, 50.1, 63.2, 84.4}, {1.60, 1.89, 1.98, 2.17, 2.34},
+                                   0.3, 11.9, 0.714, 0.4};
+
+int sampled_cluster(const amm_batch* b, const std::vector<std::pair<int, int>>& sizes) {
+  const SampledCost& k = b->cfg.nvec == 4 ? kSampled4 : kSampled8;
+  const double it = (double)std::min<int64_t>(b->cfg.max_iter, 20);
+  const double exact = (double)exact_of_sampled(b->cfg, (int64_t)it);
+  int best = 0;
+  double best_us = 0.0;
+  for (const auto& size : sizes) {
+    const int cl = size.first;  // CTAs of a cluster, and the clusters
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+    for (int i = 0; i < size.second; ++i) free_at.push(0.0);
+    double end = 0.0;
+    for (const int32_t i : b->order) {
+      const Mat& x = b->mats[i];
+      int w = 0;
+      while (w < 4 && 128 << w < x.m) ++w;
+      const double teams = (double)((16 >> w) * cl);
+      const double fixed = k.fixed[w] + (cl > 1 ? k.join + k.join_row * (double)(cl << w) : 0.0);
+      const double groups = (double)x.n / (4.0 * teams);
+      const double picked = k.distinct * (double)x.c / (4.0 * teams);
+      const double us = (it + 1.0) * fixed + (exact + 0.1) * groups * k.group[w] +
+                        (it - exact) * (k.draw + picked * k.group[w]);
+      const double done = free_at.top() + us;
+      free_at.pop();
+      free_at.push(done);
+      end = std::max(end, done);
+    }
+    if (best == 0 || end < best_us) {
+      best = cl;
+      best_us = end;
+    }
+  }
+  return best;
+}
+
+// Whether the wide launch may take a matrix: in a sampled batch of blocks one with picks enough that
+// the order of its sums is rounding alone.
+bool wide_may_take(const amm_batch* b, int32_t i) {
+  return !b->amm || b->cfg.nvec == 1 || b->mats[i].c >= 16 * b->cfg.nvec;
+}
+
 // Wide-cluster plan for a batch of uneven matrices.  With one cluster size for all, a matrix
 // whose work alone, on one cluster, exceeds an even share of the whole batch per cluster sets
 // the run's time (the queue hands it out first, but nothing can help with it).  Those leading
@@ -1992,7 +2047,9 @@ void plan_wide(amm_batch* b) {
   const double share = 0.75 * total / (double)b->nsm;
   auto work = [&](int k) { return b->cost[b->order[k]]; };
   int nwide = 0;
-  while (nwide < b->count && work(nwide) > (double)b->cluster * share) ++nwide;
+  while (nwide < b->count && work(nwide) > (double)b->cluster * share &&
+         wide_may_take(b, b->order[nwide]))
+    ++nwide;
   if (nwide == 0) return;
   int wcl = 0;
   for (int cl : amm::batch::kClusterSizes) {
@@ -2018,7 +2075,7 @@ void plan_wide(amm_batch* b) {
 // Tile-shape autotuner: every (columns per group, cluster size) pair with the requested K runs
 // the whole batch for up to 20 iterations (enough for the per-matrix set-up, which favours
 // larger clusters, to weigh as it does in a real run); the fastest of two timed runs (CUDA
-// events) is kept for the context.
+// events) is kept for the context.  A sampled batch of blocks is not timed (sampled_cluster).
 int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaStream_t s) {
   if (b->variant >= 0) return AMM_OK;
   int best = -1, best_cl = 1, best_grid = 0;
@@ -2027,8 +2084,10 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   BATCH_CUDA(cudaEventCreate(&e0));
   BATCH_CUDA(cudaEventCreate(&e1));
   const int n_var = (int)(sizeof(amm::batch::kVariants) / sizeof(amm::batch::kVariants[0]));
-  // the candidates; a single one (tile and cluster size fixed by the caller) is taken untimed
+  // the candidates; a single one (tile and cluster size fixed by the caller, or a sampled batch of
+  // blocks) is taken untimed
   std::vector<std::tuple<int, int, int>> cand;  // (variant, cluster size, grid)
+  const bool sampled_blocks = b->amm && b->cfg.nvec > 1;
   for (int v = 0; v < n_var; ++v) {
     if (amm::batch::kVariants[v].K != b->cfg.nvec) continue;
     if (amm::batch::kVariants[v].tc && (b->amm || !b->d_tmaps)) continue;  // exact-only, maps
@@ -2036,21 +2095,33 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
     // exact one is tried
     if (b->ntiles > 0 && !b->amm && b->d_tmaps && b->cfg.nvec == 8 && !amm::batch::kVariants[v].tc)
       continue;
-    if (b->cfg.tile_gc > 0 && amm::batch::kVariants[v].GC != b->cfg.tile_gc) continue;
+    const int gc = b->cfg.tile_gc > 0 ? b->cfg.tile_gc : sampled_blocks ? 4 : 0;
+    if (gc > 0 && amm::batch::kVariants[v].GC != gc) continue;
     for (int cl : amm::batch::kClusterSizes) {
       if (b->cfg.cluster > 0 && cl != b->cfg.cluster) continue;
       const int grid = persistent_grid(b, v, cl);
       if (grid > 0) cand.emplace_back(v, cl, grid);
     }
   }
+  const bool fixed = cand.size() == 1;
+  if (sampled_blocks && cand.size() > 1) {
+    std::vector<std::pair<int, int>> sizes;
+    for (const auto& cd : cand) sizes.emplace_back(std::get<1>(cd), std::get<2>(cd) / std::get<1>(cd));
+    const int cl = sampled_cluster(b, sizes);
+    for (const auto& cd : std::vector<std::tuple<int, int, int>>(cand))
+      if (std::get<1>(cd) == cl) cand.assign(1, cd);
+  }
   if (cand.size() == 1) {
     b->variant = std::get<0>(cand[0]);
     b->cluster = std::get<1>(cand[0]);
     b->grid = std::get<2>(cand[0]);
-    plan_wide(b);  // only with wide = 1 (the cluster size is the caller's); untimed
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    return AMM_OK;
+    plan_wide(b);  // untimed with wide = 1, and where the cluster size is the caller's
+    if (fixed || b->wide_count == 0 || b->cfg.wide == 1) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      return AMM_OK;
+    }
+    b->variant = -1;  // the plan is timed below against the run without it
   }
   for (const auto& cd : cand) {
     const int v = std::get<0>(cd), cl = std::get<1>(cd), grid = std::get<2>(cd);
@@ -2172,30 +2243,16 @@ static bool encode_tensor_maps(const std::vector<Mat>& ms, std::vector<CUtensorM
   return true;
 }
 
-// Exact products of a run (a tolerance may stop it earlier: 16 are counted then).
+// Products of an exact run (a tolerance may stop it earlier: 16 are counted then).
 static double exact_products(const amm_batch_config& cfg) {
-  const int64_t it = cfg.max_iter;
-  if (cfg.c_divisor > 0) {
-    if (cfg.vr_period <= 0) return 0.0;
-    return (double)(it / cfg.vr_period + (it % cfg.vr_period != 0 ? 1 : 0));
-  }
-  return (double)(cfg.tol > 0.0 ? std::min<int64_t>(it, 16) : it);
-}
-
-// Estimated clocks of one SM for a run's products of a matrix through A: 11 bytes of A a clock on the
-// tensor-core product, 8.5 on the CUDA-core one (C4, measured).
-static double direct_clocks(const Mat& x, const amm_batch_config& cfg) {
-  const double rate = cfg.nvec == 8 && cfg.c_divisor == 0 ? 11.0 : 8.5;
-  const double p = cfg.c_divisor > 0
-                       ? exact_products(cfg) + (double)cfg.max_iter / (double)cfg.c_divisor
-                       : exact_products(cfg);
-  return p * 4.0 * (double)x.m * (double)x.n / rate;
+  return (double)(cfg.tol > 0.0 ? std::min<int64_t>(cfg.max_iter, 16) : cfg.max_iter);
 }
 
 // Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which forming C
 // (2500 clocks per 128 x 128 tile and 64 columns) and the products with it (m·m·nvec FMAs at 128 a
-// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only with the tile shape
-// left to the library (a fixed one asks for its product) and an even block; none without `with_c`.
+// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only in exact batches (the
+// order of a sampled batch's sums is fixed, see sampled_cluster), with the tile shape left to the
+// library (a fixed one asks for its product) and an even block; none without `with_c`.
 // Returns C's floats in all; `cost`: estimated clocks per matrix.
 static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c,
                          std::vector<double>& cost) {
@@ -2206,12 +2263,15 @@ static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool
     Mat& x = ms[i];
     x.C = nullptr;
     x.ldc = (x.m + 3) / 4 * 4;
-    const double direct = p * 4.0 * (double)x.m * (double)x.n /
-                          (cfg.nvec == 8 && cfg.c_divisor == 0 ? 11.0 : 8.5);
+    cost[i] = (double)x.m * (double)x.n;
+    if (cfg.c_divisor > 0) continue;
+    // clocks of one SM through A: 11 bytes of A a clock on the tensor-core product, 8.5 on the CUDA-core
+    // one (measured on the 512-matrix batch)
+    const double direct = p * 4.0 * cost[i] / (cfg.nvec == 8 ? 11.0 : 8.5);
     const double t = (double)((x.m + 127) / 128), chunks = (double)((x.n + 63) / 64);
     const double form = t * (t + 1) / 2 * chunks * 2500.0;
     const double by_c = p * (double)x.m * (double)x.m * (double)cfg.nvec / 96.0;
-    cost[i] = direct_clocks(x, cfg);
+    cost[i] = direct;
     if (with_c && cfg.tile_gc == 0 && cfg.nvec % 2 == 0 && form + by_c < 0.8 * direct) {
       x.C = reinterpret_cast<float*>(1);  // placed by place_gram
       floats += (int64_t)x.ldc * x.ldc;
