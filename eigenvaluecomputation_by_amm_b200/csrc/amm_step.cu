@@ -594,7 +594,10 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
     const int ngroups = (nb + GC - 1) / GC;
 
     // the groups of this step already in the ring (issued at the end of the previous step on the
-    // predicted list, or left there by it); a misprediction is drained and the ring moves on
+    // predicted list, or left there by it); a misprediction is drained and the ring moves on.  No
+    // thread may wait for a new group before the drain is over: where the drained groups filled the
+    // ring, a new one takes the stage of one still landing, and a wait for that stage's next phase
+    // would see the phase before it complete and go through at once.
     int pre = 0;
     {
       const int pn = pre_s[0];
@@ -602,18 +605,22 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
         if (pre_s[1] == key) {
           pre = pn;
         } else {
+          bool drained = true;
           if (warp == iw && lane == 0) {
             int sg = s_cur;
             uint32_t ph = ph_cur;
-            for (int k = 0; k < pn; ++k) {
-              mbar_wait_bounded(&full[sg], ph);
+            for (int k = 0; k < pn && drained; ++k) {
+              drained = mbar_wait_bounded(&full[sg], ph);
               if (++sg == NS) {
                 sg = 0;
                 ph ^= 1u;
               }
             }
           }
-          __syncwarp();
+          if (named_barrier_or(1, T, !drained)) {
+            leave(true, i - a.iter + 1);
+            return;
+          }
           advance(pn);
         }
       }
