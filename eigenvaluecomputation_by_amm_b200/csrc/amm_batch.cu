@@ -14,10 +14,9 @@
 // ring that keeps two or more groups in flight), forms the K·GC partial dots A_jᵀX over its
 // rows, reduces them across the team (warp butterfly, then shared memory for teams wider than a
 // warp) and accumulates Y += A_j·(A_jᵀX): the fused single-pass product of the main kernel.
-// Where it pays (plan_gram) the exact products of blocks of 4 or 8 go through C = A·Aᵀ, formed once
-// per run on tcgen05 (amm_gram.cu), as C·X (cx_product).  Exact batches of 8 vectors take a
-// tensor-core form of the product through A otherwise (TF32 mma.sync with a hi + lo split, column
-// tiles copied by TMA; see batch_kernel).
+// Exact batches of 8 vectors take a tensor-core form of that product (TF32 mma.sync with a hi + lo
+// split, column tiles copied by TMA; see batch_kernel) and, where it pays (plan_gram), go through
+// C = A·Aᵀ, formed once per run on tcgen05 (amm_gram.cu), as C·X (cx_product).
 // After the pass the team partials of Y are summed in a fixed order, the Gram matrices
 // G = YᵀY and H = XᵀY are reduced in FP64, X <- Y·R⁻¹ (Cholesky QR), and every rr_period
 // iterations (and at the end) H is diagonalised by a warp-parallel cyclic Jacobi in FP64: its
@@ -785,9 +784,8 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 }
 
 // Y = C·X over this team's share of C's columns (C = A·Aᵀ, ldc x ldc, zeros past m), this thread's
-// rows r0 .. r0 + 3, for an even number of vectors: per column one 16-byte load of C (coalesced
-// over the team, four columns ahead in registers) against X's row (broadcast loads: `xrow`, see yq,
-// or without it the interleaved pairs of Xs), in packed FP32 FMAs.  Bounded by the FMAs and by an
+// rows r0 .. r0 + 3: per column one 16-byte load of C (coalesced over the team, four columns ahead in
+// registers) against X's row (broadcast loads from `xrow`, see yq), in packed FP32 FMAs.  Bounded by the FMAs and by an
 // SM's share of the L2 (16 packed FMAs per 16 bytes).  The sums are taken in runs of 16 columns, added
 // up in this thread's slot of shared memory (`slots`, [value / 4][thread]): one FP32 chain over a
 // team's whole share made the rounding of Y the largest error of λ where the eigenvector sits on
@@ -795,8 +793,7 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 // registers do not compete with the other product loops'.
 template <int K>
 __device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, const float* xrow,
-                                        const float* Xs, float4* slots, int r0, int g0,
-                                        int gstep) {
+                                        float4* slots, int r0, int g0, int gstep) {
   constexpr int KP = K / 2;
   float2 run[4][KP];
 #pragma unroll
@@ -835,18 +832,11 @@ __device__ __noinline__ void cx_product(const float* __restrict__ C, int ldc, co
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         float2 x[KP];
-        const int k = 4 * g + j;
-        if (xrow) {
 #pragma unroll
-          for (int p = 0; p < KP; p += 2) {
-            const float4 v = reinterpret_cast<const float4*>(xrow)[yq<K>(g, j * (K / 4) + p / 2)];
-            x[p] = make_float2(v.x, v.y);
-            x[p + 1] = make_float2(v.z, v.w);
-          }
-        } else {
-#pragma unroll
-          for (int p = 0; p < KP; ++p)
-            x[p] = *reinterpret_cast<const float2*>(Xs + p * 2 * kMaxRows + 2 * k);
+        for (int p = 0; p < KP; p += 2) {
+          const float4 v = reinterpret_cast<const float4*>(xrow)[yq<K>(g, j * (K / 4) + p / 2)];
+          x[p] = make_float2(v.x, v.y);
+          x[p + 1] = make_float2(v.z, v.w);
         }
         const float ce[4] = {c[j].x, c[j].y, c[j].z, c[j].w};
 #pragma unroll
@@ -1244,14 +1234,14 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // ---- Y = C·X (or its AMM estimate): the fused pass over the columns (team-local) ----
       const bool rows = r0 < m;
       int buf = 0;
-      const bool by_c = K % 2 == 0 && M.C != nullptr;  // the product as C·X (exact batches)
+      const bool by_c = TC && M.C != nullptr;  // the product as C·X
       if (by_c) {
         // (nothing that this kernel keeps in registers is passed to an out-of-line function by
         // address: it would live in local memory, and the L1 left beside the shared memory is
         // streamed through by the products)
-        if constexpr (K % 2 == 0) {
-          cx_product<K>(M.C, M.ldc, TC ? reinterpret_cast<const float*>(smem + SL::xrow) : nullptr,
-                        Xs, reinterpret_cast<float4*>(yred), r0, gteam, NTG);
+        if constexpr (TC) {
+          cx_product<K>(M.C, M.ldc, reinterpret_cast<const float*>(smem + SL::xrow),
+                        reinterpret_cast<float4*>(yred), r0, gteam, NTG);
           memo_load<K>(yred, t, Y);
         }
         __syncthreads();  // the slots lie where Y is copied next
@@ -2091,10 +2081,9 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   for (int v = 0; v < n_var; ++v) {
     if (amm::batch::kVariants[v].K != b->cfg.nvec) continue;
     if (amm::batch::kVariants[v].tc && (b->amm || !b->d_tmaps)) continue;  // exact-only, maps
-    // with products as C·X the tile shape matters to the other matrices alone: only the best
-    // exact one is tried
-    if (b->ntiles > 0 && !b->amm && b->d_tmaps && b->cfg.nvec == 8 && !amm::batch::kVariants[v].tc)
-      continue;
+    // products as C·X are in the tensor-core kernel, whose product through A is the fastest exact one
+    // as well (42 sizes with m 64-2048, n = m/4 .. 5m, 16 and 148 or 296 matrices)
+    if (b->ntiles > 0 && !amm::batch::kVariants[v].tc) continue;
     const int gc = b->cfg.tile_gc > 0 ? b->cfg.tile_gc : sampled_blocks ? 4 : 0;
     if (gc > 0 && amm::batch::kVariants[v].GC != gc) continue;
     for (int cl : amm::batch::kClusterSizes) {
@@ -2250,9 +2239,11 @@ static double exact_products(const amm_batch_config& cfg) {
 
 // Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which forming C
 // (2500 clocks per 128 x 128 tile and 64 columns) and the products with it (m·m·nvec FMAs at 128 a
-// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only in exact batches (the
-// order of a sampled batch's sums is fixed, see sampled_cluster), with the tile shape left to the
-// library (a fixed one asks for its product) and an even block; none without `with_c`.
+// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only in exact batches of 8
+// vectors with the tile shape left to the library (a fixed one asks for its product): the order of a
+// sampled batch's sums is fixed (see sampled_cluster), and the FP32 products of 4 vectors are the more
+// accurate ones (λ's rms error against FP64 over 214 matrices: 6.6e-8 through A, 7.8e-8 through C; 8
+// vectors: 1.4e-7 through A, 7.7e-8 through C).  None without `with_c`.
 // Returns C's floats in all; `cost`: estimated clocks per matrix.
 static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c,
                          std::vector<double>& cost) {
@@ -2264,15 +2255,14 @@ static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool
     x.C = nullptr;
     x.ldc = (x.m + 3) / 4 * 4;
     cost[i] = (double)x.m * (double)x.n;
-    if (cfg.c_divisor > 0) continue;
-    // clocks of one SM through A: 11 bytes of A a clock on the tensor-core product, 8.5 on the CUDA-core
-    // one (measured on the 512-matrix batch)
-    const double direct = p * 4.0 * cost[i] / (cfg.nvec == 8 ? 11.0 : 8.5);
+    if (cfg.c_divisor > 0 || cfg.nvec != 8) continue;
+    // clocks of one SM through A: 11 bytes of A a clock (measured on the 512-matrix batch)
+    const double direct = p * 4.0 * cost[i] / 11.0;
     const double t = (double)((x.m + 127) / 128), chunks = (double)((x.n + 63) / 64);
     const double form = t * (t + 1) / 2 * chunks * 2500.0;
-    const double by_c = p * (double)x.m * (double)x.m * (double)cfg.nvec / 96.0;
+    const double by_c = p * (double)x.m * (double)x.m * 8.0 / 96.0;
     cost[i] = direct;
-    if (with_c && cfg.tile_gc == 0 && cfg.nvec % 2 == 0 && form + by_c < 0.8 * direct) {
+    if (with_c && cfg.tile_gc == 0 && form + by_c < 0.8 * direct) {
       x.C = reinterpret_cast<float*>(1);  // placed by place_gram
       floats += (int64_t)x.ldc * x.ldc;
       cost[i] += by_c - direct;  // (C is formed by a launch of its own)
@@ -2339,12 +2329,15 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
     cols += x.n;
   }
   std::vector<double> cost;
-  const int64_t c_floats = plan_gram(ms, *cfg, with_c, cost);
+  Guard g(device);
+  // tensor maps when the tensor-core kernel can run: exact, 8 vectors
+  std::vector<CUtensorMap> tmaps;
+  const bool with_tmaps = !amm_mode && cfg->nvec == 8 && encode_tensor_maps(ms, tmaps);
+  const int64_t c_floats = plan_gram(ms, *cfg, with_c && with_tmaps, cost);
   amm_batch* b = new amm_batch();
   b->device = device;
   b->cfg = *cfg;
   b->count = count;
-  Guard g(device);
   if (c_floats > 0) {
     const cudaError_t ce = cudaMalloc(&b->c_mem, sizeof(float) * (size_t)c_floats);
     if (ce != cudaSuccess) {
@@ -2388,8 +2381,7 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
   const bool with_vr = amm_mode && cfg->vr_period > 0;
   const size_t vr_floats = (size_t)amm::batch::kVrSlot * amm::batch::kMaxRows * cfg->nvec;
   const size_t o_vr = with_vr ? carve(sizeof(float) * vr_floats * b->nsm, 256) : 0;
-  // tensor maps (64-byte aligned each) when the tensor-core kernel can run: exact, 8 vectors
-  const bool with_tmaps = !amm_mode && cfg->nvec == 8 && encode_tensor_maps(ms, b->h_tmaps);
+  b->h_tmaps.swap(tmaps);  // (64-byte aligned each on the device)
   const size_t o_tiles = carve(sizeof(amm::batch::GramTile) * (tiles.empty() ? 1 : tiles.size()), 256);
   const size_t o_tmaps = with_tmaps ? carve(sizeof(CUtensorMap) * count, 256) : 0;
   cudaError_t e = cudaMalloc(&b->mem, bytes);

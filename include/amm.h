@@ -267,8 +267,8 @@ typedef struct amm_batch_config {
   double tol;         /* stop when ‖C·v − λ_max·v‖ <= tol·λ_max (v: the top Ritz vector)  */
   uint64_t seed;      /* start block (counter-based hash of seed, matrix, row, vector)    */
   int32_t use_graph;  /* replay the launch from a CUDA graph                             */
-  int32_t tile_gc;    /* columns per group; 0 lets the library choose, and lets blocks of 4 */
-                      /* or 8 take their exact products as C·X (C = A·Aᵀ formed every run,  */
+  int32_t tile_gc;    /* columns per group; 0 lets the library choose, and lets exact runs  */
+                      /* of 8 vectors take their products as C·X (C = A·Aᵀ formed every run, */
                       /* m·m floats per such matrix) where that is less work; 8 (nvec = 8,  */
                       /* exact products only) is the tensor-core product: TF32 mma.sync   */
                       /* with a hi/lo split of A, X and AᵀX (about FP32 accuracy)          */
