@@ -31,7 +31,6 @@
 #include <cstdint>
 #include <cstring>
 #include <functional>
-#include <map>
 #include <queue>
 #include <tuple>
 #include <utility>
@@ -87,6 +86,7 @@ struct Args {
   // tensor-core kernel: one tensor map per matrix (FP32 {m rows, n columns}, 32 x 8 boxes,
   // 128-byte swizzle, zero fill outside the matrix), encoded on the host
   const CUtensorMap* tmaps;
+  int32_t use_c;  // products as C·X where a matrix has its C (0: every product reads A)
 };
 
 // A shared-memory float4 load the compiler keeps in place (X is re-read per column group
@@ -1144,7 +1144,7 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
           for (int j = 0; j < K; ++j)
             *reinterpret_cast<float4*>(Xs + xs_idx<K, true>(j, r0)) =
                 make_float4(X[0][j], X[1][j], X[2][j], X[3][j]);
-          if (M.C) y_store<K>(reinterpret_cast<float*>(smem + SL::xrow), t, X);
+          if (a.use_c && M.C) y_store<K>(reinterpret_cast<float*>(smem + SL::xrow), t, X);
         } else if constexpr (K % 2 == 0) {  // interleaved pairs
 #pragma unroll
           for (int j = 0; j < K; j += 2)
@@ -1234,7 +1234,7 @@ __global__ void __launch_bounds__(kThreads, 1) batch_kernel(const __grid_constan
       // ---- Y = C·X (or its AMM estimate): the fused pass over the columns (team-local) ----
       const bool rows = r0 < m;
       int buf = 0;
-      const bool by_c = TC && M.C != nullptr;  // the product as C·X
+      const bool by_c = TC && a.use_c && M.C != nullptr;  // the product as C·X
       if (by_c) {
         // (nothing that this kernel keeps in registers is passed to an out-of-line function by
         // address: it would live in local memory, and the L1 left beside the shared memory is
@@ -1739,7 +1739,6 @@ struct amm_batch {
   amm_batch_config cfg{};
   int64_t count = 0;
   std::vector<Mat> mats;
-  std::vector<int32_t> order;
   int64_t vec_len = 0;
   int64_t total_cols = 0;
   int64_t n_states = 0;
@@ -1748,12 +1747,14 @@ struct amm_batch {
   float* c_mem = nullptr;
   amm::batch::GramTile* d_tiles = nullptr;
   int ntiles = 0;
-  std::vector<double> cost;  // estimated clocks of a run per matrix, for the order and the plan (sampled
-                             // batches: m·n)
+  // costs per matrix and the processing order they give (largest first), [0] with every product
+  // through A, [1] with products as C·X where planned
+  std::vector<double> cost[2];
+  std::vector<int32_t> order[2];
   // device memory (one allocation)
   void* mem = nullptr;
   Mat* d_mats = nullptr;
-  int32_t* d_order = nullptr;
+  int32_t* d_order = nullptr;  // both orders, one after the other
   uint32_t* d_queue = nullptr;
   int64_t* d_col_start = nullptr;
   float** d_grads = nullptr;
@@ -1771,6 +1772,7 @@ struct amm_batch {
   int rec_products = 0;
   int variant = -1;  // chosen tile shape (index into kVariants)
   int cluster = 1;   // CTAs per matrix (cluster size)
+  bool use_c = false;  // products as C·X where planned
   int grid = 0;      // CTAs of the persistent launch for that cluster size
   // The heaviest matrices on a wide-cluster launch (wide_count 0: one launch per run): it takes
   // the first wide_count matrices of the order on clusters of wide_cluster CTAs, then joins
@@ -1780,7 +1782,6 @@ struct amm_batch {
   int wide_grid = 0;
   int narrow_grid = 0;
   float wide_ms = 0.f;   // the plan's time in the autotuner (0: not timed)
-  std::map<std::pair<int, int>, float> tune_ms;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t gexec = nullptr;
   cudaStream_t cap = nullptr;
@@ -1851,13 +1852,13 @@ int persistent_grid(amm_batch* b, int variant, int cl) {
 }
 
 // Start of a run: both work-list counters zeroed and, in AMM mode, the seeded states restored
-// (every run draws the same picks).
-int run_prologue(amm_batch* b, cudaStream_t s, bool gram = true) {
+// (every run draws the same picks); C formed where products go through it (gram).
+int run_prologue(amm_batch* b, cudaStream_t s, bool gram) {
   BATCH_CUDA(cudaMemsetAsync(b->d_queue, 0, 4 * sizeof(uint32_t), s));
   if (b->amm)
     BATCH_CUDA(cudaMemcpyAsync(b->d_states, b->d_states0, sizeof(uint32_t) * b->n_states,
                                cudaMemcpyDeviceToDevice, s));
-  if (gram && b->ntiles > 0)
+  if (gram)
     BATCH_CUDA(amm::batch::launch_gram(b->d_mats, b->d_tiles, b->ntiles, b->d_queue + 2, b->nsm, s));
   return AMM_OK;
 }
@@ -1867,7 +1868,7 @@ int run_prologue(amm_batch* b, cudaStream_t s, bool gram = true) {
 // stream, so that it starts on the SMs that launch leaves free.
 int launch_kernel(amm_batch* b, int variant, int cl, int grid, double* d_lam, float* d_vec,
                   int32_t* d_iters, int max_iter, const int32_t* order, int count,
-                  const int32_t* order0, int count0, bool dependent, cudaStream_t s,
+                  const int32_t* order0, int count0, bool dependent, bool use_c, cudaStream_t s,
                   int vr_base = 0) {
   const auto& V = amm::batch::kVariants[variant];
   const int sm = amm::batch::smem_bytes(V, b->amm);
@@ -1897,6 +1898,7 @@ int launch_kernel(amm_batch* b, int variant, int cl, int grid, double* d_lam, fl
   a.rec_products = b->rec_products;
   a.col_start = b->d_col_start;
   a.tmaps = b->d_tmaps;
+  a.use_c = use_c ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(amm::batch::kThreads, 1, 1);
@@ -1917,14 +1919,19 @@ int launch_kernel(amm_batch* b, int variant, int cl, int grid, double* d_lam, fl
   return AMM_OK;
 }
 
-// A run as one launch over the order list (or a slice of it).
+// The device's order list for products with or without C.
+const int32_t* order_of(const amm_batch* b, bool use_c) {
+  return b->d_order + (use_c ? b->count : 0);
+}
+
+// A run as one launch over the order list (or a slice of it); gram: C is formed first.
 int launch(amm_batch* b, int variant, int cl, int grid, double* d_lam, float* d_vec,
-           int32_t* d_iters, int max_iter, const int32_t* order, int count, cudaStream_t s,
-           bool gram = true) {
+           int32_t* d_iters, int max_iter, const int32_t* order, int count, bool use_c, bool gram,
+           cudaStream_t s) {
   const int rc = run_prologue(b, s, gram);
   if (rc) return rc;
   return launch_kernel(b, variant, cl, grid, d_lam, d_vec, d_iters, max_iter, order, count,
-                       nullptr, 0, false, s);
+                       nullptr, 0, false, use_c, s);
 }
 
 // A run with the wide-cluster plan: the wide launch takes the heaviest matrices first, the
@@ -1932,22 +1939,23 @@ int launch(amm_batch* b, int variant, int cl, int grid, double* d_lam, float* d_
 // of the order list.
 int launch_wide(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, int max_iter,
                 cudaStream_t s) {
-  int rc = run_prologue(b, s);
+  int rc = run_prologue(b, s, b->use_c);
   if (rc) return rc;
-  const int32_t* rest = b->d_order + b->wide_count;
+  const int32_t* first = order_of(b, b->use_c);
+  const int32_t* rest = first + b->wide_count;
   const int nrest = (int)b->count - b->wide_count;
   rc = launch_kernel(b, b->variant, b->wide_cluster, b->wide_grid, d_lam, d_vec, d_iters,
-                     max_iter, rest, nrest, b->d_order, b->wide_count, false, s);
+                     max_iter, rest, nrest, first, b->wide_count, false, b->use_c, s);
   if (rc) return rc;
   return launch_kernel(b, b->variant, b->cluster, b->narrow_grid, d_lam, d_vec, d_iters,
-                       max_iter, rest, nrest, nullptr, 0, true, s, b->wide_grid);
+                       max_iter, rest, nrest, nullptr, 0, true, b->use_c, s, b->wide_grid);
 }
 
 // The run of the chosen plan.
 int launch_run(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaStream_t s) {
   if (b->wide_count > 0) return launch_wide(b, d_lam, d_vec, d_iters, (int)b->cfg.max_iter, s);
   return launch(b, b->variant, b->cluster, b->grid, d_lam, d_vec, d_iters,
-                (int)b->cfg.max_iter, b->d_order, (int)b->count, s);
+                (int)b->cfg.max_iter, order_of(b, b->use_c), (int)b->count, b->use_c, b->use_c, s);
 }
 
 // Exact products of `it` products of a sampled run with variance reduction.
@@ -1989,7 +1997,7 @@ int sampled_cluster(const amm_batch* b, const std::vector<std::pair<int, int>>& 
     std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
     for (int i = 0; i < size.second; ++i) free_at.push(0.0);
     double end = 0.0;
-    for (const int32_t i : b->order) {
+    for (const int32_t i : b->order[0]) {
       const Mat& x = b->mats[i];
       int w = 0;
       while (w < 4 && 128 << w < x.m) ++w;
@@ -2030,15 +2038,17 @@ void plan_wide(amm_batch* b) {
   b->wide_count = 0;
   if (!amm::pdl_enabled() || b->cfg.wide < 0 || b->count < 2) return;
   if (b->cfg.cluster > 0 && b->cfg.wide == 0) return;
+  const std::vector<double>& cost = b->cost[b->use_c];
+  const std::vector<int32_t>& order = b->order[b->use_c];
   double total = 0.0;
-  for (const double c : b->cost) total += c;
+  for (const double c : cost) total += c;
   // work per SM of an even split, with a margin: the per-CTA rate falls with the row count,
   // so the heaviest matrices are also the slowest per element
   const double share = 0.75 * total / (double)b->nsm;
-  auto work = [&](int k) { return b->cost[b->order[k]]; };
+  auto work = [&](int k) { return cost[order[k]]; };
   int nwide = 0;
   while (nwide < b->count && work(nwide) > (double)b->cluster * share &&
-         wide_may_take(b, b->order[nwide]))
+         wide_may_take(b, order[nwide]))
     ++nwide;
   if (nwide == 0) return;
   int wcl = 0;
@@ -2065,10 +2075,13 @@ void plan_wide(amm_batch* b) {
 // Tile-shape autotuner: every (columns per group, cluster size) pair with the requested K runs
 // the whole batch for up to 20 iterations (enough for the per-matrix set-up, which favours
 // larger clusters, to weigh as it does in a real run); the fastest of two timed runs (CUDA
-// events) is kept for the context.  A sampled batch of blocks is not timed (sampled_cluster).
+// events) is kept for the context.  A sampled batch of blocks is not timed (sampled_cluster).  Where
+// products are planned as C·X and a tolerance ends the run, the run without C is timed too: whether
+// forming C pays depends on how many products it takes to converge.
 int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaStream_t s) {
   if (b->variant >= 0) return AMM_OK;
   int best = -1, best_cl = 1, best_grid = 0;
+  bool best_c = false;
   float best_ms = 0.f;
   cudaEvent_t e0, e1;
   BATCH_CUDA(cudaEventCreate(&e0));
@@ -2076,7 +2089,7 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   const int n_var = (int)(sizeof(amm::batch::kVariants) / sizeof(amm::batch::kVariants[0]));
   // the candidates; a single one (tile and cluster size fixed by the caller, or a sampled batch of
   // blocks) is taken untimed
-  std::vector<std::tuple<int, int, int>> cand;  // (variant, cluster size, grid)
+  std::vector<std::tuple<int, int, int, bool>> cand;  // (variant, cluster size, grid, with C)
   const bool sampled_blocks = b->amm && b->cfg.nvec > 1;
   for (int v = 0; v < n_var; ++v) {
     if (amm::batch::kVariants[v].K != b->cfg.nvec) continue;
@@ -2089,7 +2102,8 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
     for (int cl : amm::batch::kClusterSizes) {
       if (b->cfg.cluster > 0 && cl != b->cfg.cluster) continue;
       const int grid = persistent_grid(b, v, cl);
-      if (grid > 0) cand.emplace_back(v, cl, grid);
+      if (grid > 0) cand.emplace_back(v, cl, grid, b->ntiles > 0);
+      if (grid > 0 && b->ntiles > 0 && b->cfg.tol > 0.0) cand.emplace_back(v, cl, grid, false);
     }
   }
   const bool fixed = cand.size() == 1;
@@ -2097,13 +2111,15 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
     std::vector<std::pair<int, int>> sizes;
     for (const auto& cd : cand) sizes.emplace_back(std::get<1>(cd), std::get<2>(cd) / std::get<1>(cd));
     const int cl = sampled_cluster(b, sizes);
-    for (const auto& cd : std::vector<std::tuple<int, int, int>>(cand))
-      if (std::get<1>(cd) == cl) cand.assign(1, cd);
+    cand.erase(std::remove_if(cand.begin(), cand.end(),
+                              [&](const auto& cd) { return std::get<1>(cd) != cl; }),
+               cand.end());
   }
   if (cand.size() == 1) {
     b->variant = std::get<0>(cand[0]);
     b->cluster = std::get<1>(cand[0]);
     b->grid = std::get<2>(cand[0]);
+    b->use_c = std::get<3>(cand[0]);
     plan_wide(b);  // untimed with wide = 1, and where the cluster size is the caller's
     if (fixed || b->wide_count == 0 || b->cfg.wide == 1) {
       cudaEventDestroy(e0);
@@ -2114,13 +2130,16 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   }
   for (const auto& cd : cand) {
     const int v = std::get<0>(cd), cl = std::get<1>(cd), grid = std::get<2>(cd);
+    const bool uc = std::get<3>(cd);
     const int iters = (int)std::min<int64_t>(b->cfg.max_iter, 20);
-    int rc = launch(b, v, cl, grid, d_lam, d_vec, d_iters, iters, b->d_order, (int)b->count, s);
+    int rc = launch(b, v, cl, grid, d_lam, d_vec, d_iters, iters, order_of(b, uc), (int)b->count, uc,
+                    uc, s);
     if (rc) return rc;
     float ms = 0.f;
     for (int rep = 0; rep < 2; ++rep) {
       BATCH_CUDA(cudaEventRecord(e0, s));
-      rc = launch(b, v, cl, grid, d_lam, d_vec, d_iters, iters, b->d_order, (int)b->count, s);
+      rc = launch(b, v, cl, grid, d_lam, d_vec, d_iters, iters, order_of(b, uc), (int)b->count, uc,
+                  uc, s);
       if (rc) return rc;
       BATCH_CUDA(cudaEventRecord(e1, s));
       BATCH_CUDA(cudaEventSynchronize(e1));
@@ -2128,11 +2147,11 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
       BATCH_CUDA(cudaEventElapsedTime(&t, e0, e1));
       ms = rep == 0 ? t : std::min(ms, t);
     }
-    b->tune_ms[{v, cl}] = ms;
     if (best < 0 || ms < best_ms) {
       best = v;
       best_cl = cl;
       best_grid = grid;
+      best_c = uc;
       best_ms = ms;
     }
   }
@@ -2144,6 +2163,12 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   b->variant = best;
   b->cluster = best_cl;
   b->grid = best_grid;
+  b->use_c = best_c;
+  if (!best_c && b->c_mem) {  // (no product reads it: use_c)
+    cudaFree(b->c_mem);
+    b->c_mem = nullptr;
+    b->ntiles = 0;
+  }
   // the wide-cluster plan, kept only if it runs faster (same iterations, best of two), or
   // untimed with wide = 1
   plan_wide(b);
@@ -2232,41 +2257,108 @@ static bool encode_tensor_maps(const std::vector<Mat>& ms, std::vector<CUtensorM
   return true;
 }
 
-// Products of an exact run (a tolerance may stop it earlier: 16 are counted then).
-static double exact_products(const amm_batch_config& cfg) {
-  return (double)(cfg.tol > 0.0 ? std::min<int64_t>(cfg.max_iter, 16) : cfg.max_iter);
+// Estimated us of one SM for a matrix: a product through A (21 KB of A a us: the tensor-core product) and
+// through C (45 KB of C a us, from L2 or HBM), each with two thirds of the idle rows of its teams (128,
+// 256, .. 2048 rows); C itself by tiles of 128 x 256 (diagonal ones of an even row block: 128 x 128), and
+// its slowest tile.
+struct GramCost {
+  double by_a, by_c, form, tile;
+};
+static GramCost gram_cost(const Mat& x) {
+  const double m = (double)x.m, n = (double)x.n;
+  double team = 128.0;
+  while (team < m) team *= 2.0;
+  const double rows = 0.65 * team + 0.35 * m;
+  const int blocks = (x.m + 127) / 128;  // of 128 rows; block ti has ti / 2 + 1 tiles
+  const double diag = (double)((blocks + 1) / 2);
+  const double full = (double)((blocks / 2 + 1) * ((blocks + 1) / 2)) - diag;
+  const double chunks = (double)((x.n + 31) / 32);
+  const double t_full = 13.2 + 1.80 * chunks, t_diag = 13.2 + 1.46 * chunks;
+  return {4.0 * rows * n / 21300.0, 4.0 * rows * m / 45000.0, diag * t_diag + full * t_full,
+          full > 0.0 ? t_full : t_diag};
 }
 
-// Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which forming C
-// (2500 clocks per 128 x 128 tile and 64 columns) and the products with it (m·m·nvec FMAs at 128 a
-// clock, 0.75 of it reached) take less than 0.8 of the products through A.  Only in exact batches of 8
-// vectors with the tile shape left to the library (a fixed one asks for its product): the order of a
-// sampled batch's sums is fixed (see sampled_cluster), and the FP32 products of 4 vectors are the more
-// accurate ones (λ's rms error against FP64 over 214 matrices: 6.6e-8 through A, 7.8e-8 through C; 8
-// vectors: 1.4e-7 through A, 7.7e-8 through C).  None without `with_c`.
-// Returns C's floats in all; `cost`: estimated clocks per matrix.
-static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c,
-                         std::vector<double>& cost) {
-  const double p = exact_products(cfg);
-  int64_t floats = 0;
-  cost.resize(ms.size());
-  for (size_t i = 0; i < ms.size(); ++i) {
-    Mat& x = ms[i];
-    x.C = nullptr;
-    x.ldc = (x.m + 3) / 4 * 4;
-    cost[i] = (double)x.m * (double)x.n;
-    if (cfg.c_divisor > 0 || cfg.nvec != 8) continue;
-    // clocks of one SM through A: 11 bytes of A a clock (measured on the 512-matrix batch)
-    const double direct = p * 4.0 * cost[i] / 11.0;
-    const double t = (double)((x.m + 127) / 128), chunks = (double)((x.n + 63) / 64);
-    const double form = t * (t + 1) / 2 * chunks * 2500.0;
-    const double by_c = p * (double)x.m * (double)x.m * 8.0 / 96.0;
-    cost[i] = direct;
-    if (with_c && cfg.tile_gc == 0 && form + by_c < 0.8 * direct) {
-      x.C = reinterpret_cast<float*>(1);  // placed by place_gram
-      floats += (int64_t)x.ldc * x.ldc;
-      cost[i] += by_c - direct;  // (C is formed by a launch of its own)
+// Estimated us of a run of p products per matrix, those of `take` through C: C's tiles over all SMs, then
+// the matrices on clusters of the best size, longest first.  An iteration costs 18 us beside its
+// product, and 6.9 ns per row and further CTA of the cluster.  (Within 4.4 % rms of 900 measured
+// runs, equal and uneven matrices, through A, through C and mixed.)
+static double gram_run_us(const std::vector<Mat>& ms, const std::vector<GramCost>& cost,
+                          const std::vector<char>& take, double p, int nsm) {
+  double form = 0.0, tile = 0.0, best = 0.0;
+  for (size_t i = 0; i < ms.size(); ++i)
+    if (take[i]) {
+      form += cost[i].form;
+      tile = std::max(tile, cost[i].tile);
     }
+  std::vector<double> us(ms.size());
+  for (int cl : amm::batch::kClusterSizes) {
+    for (size_t i = 0; i < ms.size(); ++i)
+      us[i] = p * ((take[i] ? cost[i].by_c : cost[i].by_a) / cl + 17.7 +
+                   0.0069 * (double)(cl - 1) * (double)ms[i].m);
+    std::sort(us.begin(), us.end(), std::greater<double>());
+    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+    // (of 148 SMs 33 clusters of 4 and 15 of 8 are resident)
+    const int clusters = std::max(1, (cl > 2 ? 9 * nsm / 10 : nsm) / cl);
+    for (int k = 0; k < clusters; ++k) free_at.push(0.0);
+    double end = 0.0;
+    for (const double u : us) {
+      const double done = free_at.top() + u;
+      free_at.pop();
+      free_at.push(done);
+      end = std::max(end, done);
+    }
+    if (cl == 1 || end < best) best = end;
+  }
+  return best + std::max(form / (double)nsm, tile);
+}
+
+// Which matrices are multiplied as C·X, C = A·Aᵀ formed once per run: those for which p products through
+// C and a share w of forming it take less than p products through A, with the w, of a few, for
+// which the run's estimate is least.  (w = 1 is right where the batch keeps every SM busy; in a small or
+// an uneven batch the time of its longest matrices counts, and forming C, unlike their products, is
+// spread over all SMs.)  Measured, 20 products of equal matrices, time through C over time through A: 296
+// of 512 x 307 1.10, 512 x 512 0.85, 512 x 2560 0.35; 148 of 1024 x 614 1.26, 1024 x 1024 0.90; 16 of 2048 x
+// 2048 0.80.  36 uneven batches of 11 to 512 matrices, m 16-2048, n 64-8192, 8 to 40 products: 0.5 % above
+// the best of every product through A, every one through C, and C by work alone, at most 17 % (11 and 55
+// matrices of up to 135 rows, where the routes lie that close); the 512-matrix batch 28.8 ms through
+// A, 13.8 through C, 12.7 by this rule.  With a tolerance 16 products are counted, and the autotuner
+// times the run without C as well.
+// Only in exact batches of 8 vectors with the tile shape left to the library (a fixed one asks for its
+// product): the order of a sampled batch's sums is fixed (see sampled_cluster), and the FP32 products
+// of 4 vectors are the more accurate ones (λ's rms error against FP64 over 214 matrices: 6.6e-8
+// through A, 7.8e-8 through C; 8 vectors: 1.4e-7 through A, 7.7e-8 through C).  None without `with_c`.
+// Returns C's floats in all; `cost`: per matrix, through A (m·n) and as planned (us a product).
+static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c, int nsm,
+                         std::vector<double> (&cost)[2]) {
+  for (auto& c : cost) c.resize(ms.size());
+  for (size_t i = 0; i < ms.size(); ++i) {
+    ms[i].C = nullptr;
+    ms[i].ldc = (ms[i].m + 3) / 4 * 4;
+    cost[0][i] = cost[1][i] = (double)ms[i].m * (double)ms[i].n;
+  }
+  if (!with_c) return 0;
+  const double p = (double)(cfg.tol > 0.0 ? std::min<int64_t>(cfg.max_iter, 16) : cfg.max_iter);
+  std::vector<GramCost> gc(ms.size());
+  for (size_t i = 0; i < ms.size(); ++i) gc[i] = gram_cost(ms[i]);
+  std::vector<char> take(ms.size(), 0), best = take, last = take;
+  double best_us = gram_run_us(ms, gc, best, p, nsm);
+  for (const double w : {1.0, 0.7, 0.5, 0.35, 0.2, 0.1}) {
+    for (size_t i = 0; i < ms.size(); ++i)
+      take[i] = w * gc[i].form + p * gc[i].by_c < p * gc[i].by_a;
+    if (take == last) continue;
+    last = take;
+    const double us = gram_run_us(ms, gc, take, p, nsm);
+    if (us < 0.99 * best_us) {
+      best_us = us;
+      best = take;
+    }
+  }
+  int64_t floats = 0;
+  for (size_t i = 0; i < ms.size(); ++i) {
+    cost[1][i] = 17.7 + (best[i] ? gc[i].by_c : gc[i].by_a);
+    if (!best[i]) continue;
+    ms[i].C = reinterpret_cast<float*>(1);  // placed by place_gram
+    floats += (int64_t)ms[i].ldc * ms[i].ldc;
   }
   return floats;
 }
@@ -2328,13 +2420,16 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
     off += x.m;
     cols += x.n;
   }
-  std::vector<double> cost;
+  std::vector<double> cost[2];
   Guard g(device);
+  int nsm = 1;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   // tensor maps when the tensor-core kernel can run: exact, 8 vectors
   std::vector<CUtensorMap> tmaps;
   const bool with_tmaps = !amm_mode && cfg->nvec == 8 && encode_tensor_maps(ms, tmaps);
-  const int64_t c_floats = plan_gram(ms, *cfg, with_c && with_tmaps, cost);
+  const int64_t c_floats = plan_gram(ms, *cfg, with_c && with_tmaps && cfg->tile_gc == 0, nsm, cost);
   amm_batch* b = new amm_batch();
+  b->nsm = nsm;
   b->device = device;
   b->cfg = *cfg;
   b->count = count;
@@ -2349,18 +2444,22 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
   std::vector<amm::batch::GramTile> tiles;
   if (b->c_mem) place_gram(ms, b->c_mem, tiles);
   b->ntiles = (int)tiles.size();
-  b->cost = cost;
   b->mats = ms;
   b->vec_len = off;
   b->total_cols = cols;
   b->n_states = nst;
   b->amm = amm_mode;
-  b->order.resize((size_t)count);
-  for (int64_t i = 0; i < count; ++i) b->order[i] = (int32_t)i;
-  // largest first (estimated clocks), ties by index: the queue then balances like LPT scheduling
-  std::stable_sort(b->order.begin(), b->order.end(),
-                   [&](int32_t x, int32_t y) { return cost[x] > cost[y]; });
-  cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, device);
+  // largest first, ties by index: the queue then balances like LPT scheduling
+  std::vector<int32_t> both((size_t)(2 * count));
+  for (int k = 0; k < 2; ++k) {
+    b->cost[k].swap(cost[k]);
+    b->order[k].resize((size_t)count);
+    for (int64_t i = 0; i < count; ++i) b->order[k][i] = (int32_t)i;
+    const std::vector<double>& c = b->cost[k];
+    std::stable_sort(b->order[k].begin(), b->order[k].end(),
+                     [&](int32_t x, int32_t y) { return c[x] > c[y]; });
+    std::copy(b->order[k].begin(), b->order[k].end(), both.begin() + k * count);
+  }
   size_t bytes = 0;
   auto carve = [&](size_t n, size_t align) {
     bytes = (bytes + align - 1) / align * align;
@@ -2369,7 +2468,7 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
     return o;
   };
   const size_t o_mats = carve(sizeof(Mat) * count, 256);
-  const size_t o_order = carve(sizeof(int32_t) * count, 256);
+  const size_t o_order = carve(sizeof(int32_t) * 2 * count, 256);
   const size_t o_queue = carve(sizeof(uint32_t) * 4, 256);
   const size_t o_cols = carve(sizeof(int64_t) * (count + 1), 256);
   const size_t o_grads = carve(sizeof(float*) * count, 256);
@@ -2407,7 +2506,7 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
   for (int64_t i = 0; i < count; ++i) cs[i + 1] = cs[i] + ms[i].n;
   e = cudaMemcpy(b->d_mats, ms.data(), sizeof(Mat) * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
-    e = cudaMemcpy(b->d_order, b->order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(b->d_order, both.data(), sizeof(int32_t) * 2 * count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess)
     e = cudaMemcpy(b->d_col_start, cs.data(), sizeof(int64_t) * (count + 1),
                    cudaMemcpyHostToDevice);
@@ -2506,7 +2605,7 @@ int amm_batch_run(amm_batch* b, double* d_lambda, float* d_vectors, int32_t* d_i
     b->g_iters = d_iters;
   }
   BATCH_CUDA(cudaGraphLaunch(b->gexec, s));
-  amm::count_launch((b->wide_count > 0 ? 2 : 1) + (b->ntiles > 0 ? 1 : 0));
+  amm::count_launch((b->wide_count > 0 ? 2 : 1) + (b->use_c ? 1 : 0));
   return AMM_OK;
 }
 
@@ -2518,10 +2617,10 @@ int amm_batch_run_each(amm_batch* b, double* d_lambda, float* d_vectors, int32_t
   int rc = autotune(b, d_lambda, d_vectors, d_iters, s);
   if (rc) return rc;
   // one single-CTA launch per matrix; each reads its matrix index from a one-entry slice of
-  // the order array
+  // the order array; C of every matrix is formed ahead of the first
   for (int64_t i = 0; i < b->count; ++i) {
     rc = launch(b, b->variant, b->cluster, b->cluster, d_lambda, d_vectors, d_iters,
-                (int)b->cfg.max_iter, b->d_order + i, 1, s, i == 0);  // (C of every matrix once)
+                (int)b->cfg.max_iter, order_of(b, false) + i, 1, b->use_c, b->use_c && i == 0, s);
     if (rc) return rc;
   }
   return AMM_OK;
