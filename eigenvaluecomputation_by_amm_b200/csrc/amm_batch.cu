@@ -2327,8 +2327,11 @@ static double gram_run_us(const std::vector<Mat>& ms, const std::vector<GramCost
 // product): the order of a sampled batch's sums is fixed (see sampled_cluster), and the FP32 products
 // of 4 vectors are the more accurate ones (λ's rms error against FP64 over 214 matrices: 6.6e-8
 // through A, 7.8e-8 through C; 8 vectors: 1.4e-7 through A, 7.7e-8 through C).  None without `with_c`.
+// Memory: all of C where an eighth of the device's free memory holds it; else the matrices that save most
+// per byte, up to a 48th, so that the caller keeps the device's memory (free_bytes, asked for once).
 // Returns C's floats in all; `cost`: per matrix, through A (m·n) and as planned (us a product).
 static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool with_c, int nsm,
+                         const std::function<size_t()>& free_bytes,
                          std::vector<double> (&cost)[2]) {
   for (auto& c : cost) c.resize(ms.size());
   for (size_t i = 0; i < ms.size(); ++i) {
@@ -2351,6 +2354,27 @@ static int64_t plan_gram(std::vector<Mat>& ms, const amm_batch_config& cfg, bool
     if (us < 0.99 * best_us) {
       best_us = us;
       best = take;
+    }
+  }
+  auto c_bytes = [&](size_t i) { return sizeof(float) * (size_t)ms[i].ldc * (size_t)ms[i].ldc; };
+  size_t planned = 0;
+  for (size_t i = 0; i < ms.size(); ++i) planned += best[i] ? c_bytes(i) : 0;
+  const size_t free_now = planned > 0 ? free_bytes() : 0;
+  if (planned > free_now / 8) {
+    std::vector<size_t> by_worth;
+    std::vector<double> worth(ms.size());
+    for (size_t i = 0; i < ms.size(); ++i) {
+      if (best[i]) by_worth.push_back(i);
+      worth[i] = (p * (gc[i].by_a - gc[i].by_c) - gc[i].form) / (double)c_bytes(i);
+    }
+    std::stable_sort(by_worth.begin(), by_worth.end(),
+                     [&](size_t x, size_t y) { return worth[x] > worth[y]; });
+    size_t room = free_now / 48;
+    std::fill(best.begin(), best.end(), 0);
+    for (const size_t i : by_worth) {
+      if (c_bytes(i) > room || !(worth[i] > 0.0)) continue;
+      room -= c_bytes(i);
+      best[i] = 1;
     }
   }
   int64_t floats = 0;
@@ -2427,7 +2451,14 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
   // tensor maps when the tensor-core kernel can run: exact, 8 vectors
   std::vector<CUtensorMap> tmaps;
   const bool with_tmaps = !amm_mode && cfg->nvec == 8 && encode_tensor_maps(ms, tmaps);
-  const int64_t c_floats = plan_gram(ms, *cfg, with_c && with_tmaps && cfg->tile_gc == 0, nsm, cost);
+  const int64_t c_floats = plan_gram(
+      ms, *cfg, with_c && with_tmaps && cfg->tile_gc == 0, nsm,
+      [] {
+        size_t free_now = 0, all = 0;
+        if (cudaMemGetInfo(&free_now, &all) != cudaSuccess) cudaGetLastError();
+        return free_now;
+      },
+      cost);
   amm_batch* b = new amm_batch();
   b->nsm = nsm;
   b->device = device;
