@@ -124,6 +124,8 @@ _SIGS = {
     "amm_batch_record": [_P, _P, _P, _I64],
     "amm_batch_set_matrices": [_P, C.POINTER(amm_batch_matrix), _I64, _P],
     "amm_batch_wide_plan": [_P, _P, _P, _P, _P],
+    "amm_batch_c_bytes": [_P],
+    "amm_batch_release_c": [_P],
     "amm_probe_bounded_waits": [_P, _P, _P],
     "amm_benchmark_product": [_P, C.c_int, C.c_int, _P, _P, _P],
     "amm_grad_lambda": [_P, _P, _P, _I64, _P],
@@ -138,6 +140,7 @@ _RET = {
     "amm_status_string": C.c_char_p,
     "amm_last_cuda_error": C.c_char_p,
     "amm_kernel_launch_count": C.c_int64,
+    "amm_batch_c_bytes": C.c_int64,
 }
 
 _lib = None

@@ -450,6 +450,14 @@ class BatchSolver:
         return {"count": int(n.value), "cluster": int(cl.value), "ctas": int(g.value),
                 "ms": float(ms.value)}
 
+    def c_bytes(self) -> int:
+        """Device memory held for C = A·Aᵀ of the matrices multiplied through it."""
+        return int(self.lib.amm_batch_c_bytes(self._b))
+
+    def release_c(self):
+        """Give C's memory back; later runs multiply through A (amm_batch_release_c)."""
+        check(self.lib.amm_batch_release_c(self._b), "amm_batch_release_c")
+
     def close(self):
         if self._b:
             self.lib.amm_batch_destroy(self._b)

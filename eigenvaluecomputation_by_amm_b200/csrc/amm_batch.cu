@@ -1745,6 +1745,7 @@ struct amm_batch {
   bool amm = false;
   // matrices multiplied as C·X: the tiles of their C = A·Aᵀ (longest first) and C's memory
   float* c_mem = nullptr;
+  int64_t c_bytes = 0;
   amm::batch::GramTile* d_tiles = nullptr;
   int ntiles = 0;
   // costs per matrix and the processing order they give (largest first), [0] with every product
@@ -1849,6 +1850,20 @@ int persistent_grid(amm_batch* b, int variant, int cl) {
   if (nclusters < 1) return 0;
   const int64_t use = std::min<int64_t>(nclusters, b->count);
   return (int)use * cl;
+}
+
+// C given back (no product reads it where use_c is off).
+void drop_c(amm_batch* b) {
+  if (b->c_mem) cudaFree(b->c_mem);
+  b->c_mem = nullptr;
+  b->ntiles = 0;
+}
+
+void drop_graph(amm_batch* b) {
+  if (b->gexec) cudaGraphExecDestroy(b->gexec);
+  if (b->graph) cudaGraphDestroy(b->graph);
+  b->gexec = nullptr;
+  b->graph = nullptr;
 }
 
 // Start of a run: both work-list counters zeroed and, in AMM mode, the seeded states restored
@@ -2164,11 +2179,7 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   b->cluster = best_cl;
   b->grid = best_grid;
   b->use_c = best_c;
-  if (!best_c && b->c_mem) {  // (no product reads it: use_c)
-    cudaFree(b->c_mem);
-    b->c_mem = nullptr;
-    b->ntiles = 0;
-  }
+  if (!best_c) drop_c(b);
   // the wide-cluster plan, kept only if it runs faster (same iterations, best of two), or
   // untimed with wide = 1
   plan_wide(b);
@@ -2465,7 +2476,8 @@ static int batch_create(amm_batch** out, const amm_batch_matrix* mats, int64_t c
   b->cfg = *cfg;
   b->count = count;
   if (c_floats > 0) {
-    const cudaError_t ce = cudaMalloc(&b->c_mem, sizeof(float) * (size_t)c_floats);
+    b->c_bytes = (int64_t)sizeof(float) * c_floats;
+    const cudaError_t ce = cudaMalloc(&b->c_mem, (size_t)b->c_bytes);
     if (ce != cudaSuccess) {
       cudaGetLastError();
       delete b;
@@ -2740,10 +2752,7 @@ int amm_batch_record(amm_batch* b, float* d_cdf, uint32_t* d_picks, int64_t prod
   b->rec_products = d_picks ? (int)products : 0;
   // the captured graph holds the launch arguments by value
   Guard g(b->device);
-  if (b->gexec) cudaGraphExecDestroy(b->gexec);
-  if (b->graph) cudaGraphDestroy(b->graph);
-  b->gexec = nullptr;
-  b->graph = nullptr;
+  drop_graph(b);
   return AMM_OK;
 }
 
@@ -2753,6 +2762,20 @@ int amm_batch_tile_choice(amm_batch* b, int32_t* k_out, int32_t* gc_out, int32_t
   *k_out = amm::batch::kVariants[b->variant].K;
   *gc_out = amm::batch::kVariants[b->variant].GC;
   if (cl_out) *cl_out = b->cluster;
+  return AMM_OK;
+}
+
+int64_t amm_batch_c_bytes(amm_batch* b) { return b && b->c_mem ? b->c_bytes : 0; }
+
+int amm_batch_release_c(amm_batch* b) {
+  if (!b) return AMM_ERR_INVALID_ARGUMENT;
+  if (!b->c_mem) return AMM_OK;
+  Guard g(b->device);
+  BATCH_CUDA(cudaDeviceSynchronize());
+  drop_graph(b);  // it forms C and reads it
+  drop_c(b);
+  b->use_c = false;
+  b->wide_count = 0;  // (planned and timed with C)
   return AMM_OK;
 }
 

@@ -332,6 +332,10 @@ int amm_batch_tile_choice(amm_batch *b, int32_t *nvec, int32_t *cols_per_group,
  * AMM_ERR_NOT_READY before the first run. */
 int amm_batch_wide_plan(amm_batch *b, int32_t *count, int32_t *cluster_size, int32_t *ctas,
                         float *ms);
+/* Device memory held for C = A·Aᵀ of the matrices multiplied through it (0: none); and C given back (once
+ * the device's work is done): the context's later runs multiply through A. */
+int64_t amm_batch_c_bytes(amm_batch *b);
+int amm_batch_release_c(amm_batch *b);
 
 /* Measurement hook: time `reps` back-to-back launches of the fused product kernel for one
  * step kind (AMM_STEP_EXACT, AMM_STEP_PREVIOUS or AMM_STEP_PROPOSED) on the bound matrix,
