@@ -2035,10 +2035,10 @@ int sampled_cluster(const amm_batch* b, const std::vector<std::pair<int, int>>& 
   return best;
 }
 
-// Whether the wide launch may take a matrix: in a sampled batch of blocks one with picks enough that
-// the order of its sums is rounding alone.
+// Whether the wide launch may take a matrix: in a sampled batch of blocks, unless the caller asked for
+// the plan, one with picks enough that the order of its sums is rounding alone.
 bool wide_may_take(const amm_batch* b, int32_t i) {
-  return !b->amm || b->cfg.nvec == 1 || b->mats[i].c >= 16 * b->cfg.nvec;
+  return !b->amm || b->cfg.nvec == 1 || b->cfg.wide == 1 || b->mats[i].c >= 16 * b->cfg.nvec;
 }
 
 // Wide-cluster plan for a batch of uneven matrices.  With one cluster size for all, a matrix

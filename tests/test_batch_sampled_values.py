@@ -26,3 +26,18 @@ def test_ritz_values_on_record(amm_lib, name):
     assert np.array_equal(np.isnan(got), np.isnan(lam)) and ok.sum() > 0.8 * len(ok)
     off = np.abs(got[ok] - lam[ok]) / lam[ok][:, :1]
     assert off.max() < 1e-6, (int(np.argmax(off.max(1))), float(off.max()))
+
+
+def test_wide_plan_that_the_caller_asked_for(amm_lib):
+    """wide = 1 plans the wide launch by work alone, also over matrices of few picks."""
+    import torch
+    from eigenvaluecomputation_by_amm_b200 import BatchSolver
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mats = [torch.randn(n, 512, device="cuda", generator=g).t() for n in [400] * 2 + [64] * 400]
+    for c_divisor in (0, 8):
+        solver = BatchSolver(mats, nvec=8, max_iter=8, tol=0.0, c_divisor=c_divisor,
+                             vr_period=4 if c_divisor else 0, tile_gc=4, cluster=1, wide=1)
+        solver.run()
+        torch.cuda.synchronize()
+        assert solver.wide_plan()["count"] == 2
+        solver.close()
