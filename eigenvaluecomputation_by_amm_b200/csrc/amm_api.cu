@@ -313,11 +313,23 @@ int single_product(amm_ctx* ctx, int method, const float* x, const float* x_memo
   if (!x || !y) return AMM_ERR_INVALID_ARGUMENT;
   DeviceGuard dg(ctx->device);
   const size_t vb = sizeof(float) * ctx->cfg.m;
-  // 16-byte aligned vectors are read by the call's first kernel, and y is written by its last; others
-  // are copied into the context first (four copies more: 52 -> 41 us a product at 4096 x 16384)
+  // 16-byte aligned vectors in this device's memory are read by the call's first kernel, and y is
+  // written by its last; others (another device's, page-locked host memory) are copied, the inputs
+  // into the context first (four copies more: 52 -> 41 us a product at 4096 x 16384).  Host memory that
+  // CUDA does not know is refused: a kernel would fault on it.
   const uintptr_t bits = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(x_memo) |
                          reinterpret_cast<uintptr_t>(y_memo);
-  const bool direct = (bits & 15) == 0;
+  bool direct = (bits & 15) == 0, y_here = true;
+  for (const void* p : {static_cast<const void*>(x), static_cast<const void*>(x_memo),
+                        static_cast<const void*>(y_memo), static_cast<const void*>(y)}) {
+    if (!p) continue;
+    cudaPointerAttributes at{};
+    AMM_CUDA(cudaPointerGetAttributes(&at, p));
+    if (at.type == cudaMemoryTypeUnregistered) return AMM_ERR_INVALID_ARGUMENT;
+    const bool here = at.type == cudaMemoryTypeDevice && at.device == ctx->device;
+    if (p == y) y_here = here && (reinterpret_cast<uintptr_t>(y) & 3) == 0;
+    direct = direct && (here || p == y);
+  }
   if (!direct) {
     if (x_memo)
       AMM_CUDA(cudaMemcpyAsync(ctx->b.x_memo, x_memo, vb, cudaMemcpyDeviceToDevice, s));
@@ -361,8 +373,9 @@ int single_product(amm_ctx* ctx, int method, const float* x, const float* x_memo
   ctx->has_run = true;
   const amm::InitMemo memo{x_memo, y_memo, ctx->x0_buf};
   rc = enqueue_call(ctx, cc, direct ? x : ctx->x0_buf, /*no_normalize=*/1, s,
-                    direct ? &memo : nullptr, y);
+                    direct ? &memo : nullptr, y_here ? y : nullptr);
   if (rc) return rc;
+  if (!y_here) AMM_CUDA(cudaMemcpyAsync(y, ctx->y_final, vb, cudaMemcpyDeviceToDevice, s));
   if (idx_out && method != amm::kMethodExact && !ext_cols && !shard) {
     if (ctx->sanity_active) {
       std::vector<uint32_t> seq(ctx->cfg.n);
