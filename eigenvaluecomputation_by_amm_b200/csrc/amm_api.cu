@@ -82,7 +82,6 @@ struct amm_ctx {
   int last_step = 0;
   bool has_run = false;
   CallCfg last_cc{};
-  std::vector<char> trace_host;  // the state, the traces and the status word, as one copy brings them
   uint32_t ext_count = 0;  // length of a caller-supplied work list (host copy read by a memcpy)
 };
 
@@ -700,9 +699,11 @@ int amm_get_trace(amm_ctx* ctx, double* eigs, double* errs, double* coss, int32_
   const size_t span =
       static_cast<size_t>(reinterpret_cast<const char*>(ctx->b.status + 1) - first);
   if (span <= kTraceSpan) {
-    ctx->trace_host.resize(span);
-    const char* host = ctx->trace_host.data();
-    AMM_CUDA(cudaMemcpyAsync(ctx->trace_host.data(), first, span, cudaMemcpyDeviceToHost, s));
+    // (a buffer of the calling thread's: several may read one context's trace at once)
+    static thread_local std::vector<char> buffer;
+    if (buffer.size() < span) buffer.resize(span);
+    char* const host = buffer.data();
+    AMM_CUDA(cudaMemcpyAsync(host, first, span, cudaMemcpyDeviceToHost, s));
     AMM_CUDA(cudaStreamSynchronize(s));
     auto at = [&](const void* dev) { return host + (static_cast<const char*>(dev) - first); };
     amm::IterState st;
