@@ -764,6 +764,7 @@ int amm_probe_bounded_waits(amm_ctx* ctx, uint32_t* result3, void* stream) {
   uint32_t* dout = reinterpret_cast<uint32_t*>(ctx->b.partials);  // scratch between steps
   AMM_CUDA(cudaMemsetAsync(ctx->b.ticket + 3, 0, sizeof(uint32_t), s));
   AMM_CUDA(amm::launch_wait_probe(ctx->b.status, ctx->b.ticket + 3, dout, s));
+  AMM_CUDA(amm::launch_packet_probe(ctx->b, dout, s));
   AMM_CUDA(cudaMemcpyAsync(result3, dout, 3 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   // the status word the step kernels set on a timeout: reported and cleared as after one
   return read_status(ctx, s);

@@ -212,6 +212,7 @@ cudaError_t launch_clock(unsigned long long* out, cudaStream_t s);
 // The failure path of the bounded waits, on purpose (one CTA; out: 3 words, see the kernel).
 cudaError_t launch_wait_probe(uint32_t* status, uint32_t* counter, uint32_t* out,
                               cudaStream_t s);
+cudaError_t launch_packet_probe(const Buffers& b, uint32_t* out, cudaStream_t s);
 cudaError_t launch_rayleigh(const float* x_in, float* x_out, const float* y, const double* vstar,
                             int m, double* out3, cudaStream_t s);
 cudaError_t launch_sample_only(const Buffers& b, int which, uint32_t* idx, cudaStream_t s);

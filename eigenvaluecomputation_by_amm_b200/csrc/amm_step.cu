@@ -1178,6 +1178,29 @@ bool step_coresident(const PanelGeom& g) {
   return per_sm >= 1;
 }
 
+// The failure path of the packet waits, on purpose (after wait_probe_kernel, whose `out` it goes on
+// with): one warp waits in each of their three forms for an epoch that nothing writes.
+__global__ void packet_probe_kernel(const uint4* p, uint32_t* status, uint32_t* out) {
+  const unsigned long long t0 = globaltimer_now();
+  const uint32_t never = packet_load(p).w + 1u;
+  uint4 v[1];
+  const int off[1] = {0};
+  bool through = packets_wait<1>(p, 0, 1, never, v);
+  through = packets_wait<1, true>(p, 0, 1, never, v) || through;
+  through = packets_wait_at<1>(p, off, 1, never, v) || through;
+  if (threadIdx.x == 0) {
+    if (through) out[1] = 1u;
+    out[2] += (uint32_t)((globaltimer_now() - t0) / 1000ull);
+    if (!through) atomicOr(status, (uint32_t)kDevTimeout);
+  }
+}
+
+cudaError_t launch_packet_probe(const Buffers& b, uint32_t* out, cudaStream_t s) {
+  packet_probe_kernel<<<1, 32, 0, s>>>(b.pk_y, b.status, out);
+  count_launch();
+  return cudaGetLastError();
+}
+
 cudaError_t launch_step(const Buffers& b, const PanelGeom& g, const CallCfg& cc, int iter,
                         int iter_end, cudaStream_t s) {
   StepArgs a{};
