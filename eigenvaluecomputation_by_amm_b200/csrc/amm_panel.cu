@@ -1213,7 +1213,8 @@ bool panel_geometry(int m, int dtype, int c, int n, int nsm, int cluster, PanelG
     --b.nstages;
     b.stage_area = b.nstages * stage;
   }
-  b.packets = step_supported(b) ? 1 : 0;
+  // (AMM_PANEL_PACKETS=0: the grid-barrier form of a device with too few SMs, for its tests)
+  b.packets = step_supported(b) && env_int("AMM_PANEL_PACKETS", 1) != 0 ? 1 : 0;
   b.smem_bytes = smem_layout(b, true).total;
   *g = b;
   return b.smem_bytes <= kSmemBudget;
