@@ -156,11 +156,15 @@ def batch_report(count=512, iters=20, check=32, modes=("exact", "amm", "amm_vr")
                               sum(1 for p in range(iters) if (p + 1) % vr == 0 or p + 1 >= iters))
             res["exact_products_per_matrix"] = exact_products if vr else 0
         if mode == "exact":
-            ach = bytes_per_product * iters / (t_one * 1e-3) / 1e9
-            res["roofline"] = {"bound": "hbm", "achieved": ach, "peak": hbm, "unit": "GB/s",
-                               "frac": ach / hbm, "peak_source": src,
-                               "note": "one read of A per product counted; matrices multiplied "
-                                       "through C = A·Aᵀ read A once per run"}
+            by_c = bs.c_bytes()  # C = A·Aᵀ of the matrices multiplied through it
+            moved = bytes_per_product + by_c if by_c else bytes_per_product * iters
+            ach = moved / (t_one * 1e-3) / 1e9
+            res["c_bytes"] = by_c
+            res["roofline"] = {"bound": "issue" if by_c else "hbm", "achieved": ach, "peak": hbm,
+                               "unit": "GB/s", "frac": ach / hbm, "peak_source": src,
+                               "note": ("A read once and C = A·Aᵀ written once per run counted; "
+                                        "bound by forming C and by FP32 issue of the products with "
+                                        "it") if by_c else "one read of A per product"}
             t_each = time_runs(bs, each=True)
             res["one_cta_launch_per_matrix_matrices_per_s"] = count * 1000.0 / t_each
         out[mode] = res
