@@ -337,10 +337,10 @@ struct Smem {
   static constexpr int tbar = align16(ctl + 16);  // uint64 [kWarps][2]: tensor-core tile copies
   static constexpr int xs = align16(tbar + kWarps * 2 * 8);              // float X[K][kMaxRows]
   static constexpr int xs_bytes = K * (TC ? kXsStrideTC : kMaxRows) * 4;
-  // one region used in turn by: the column ring during a product pass; the team partials of Y
-  // after it (yred); the block D of a sampled product with variance reduction (yred, during
-  // that product, which then keeps its columns in registers); the pick histogram of an AMM draw
-  // (hist, zeroed at the start of every draw)
+  // one region used in turn by: the column ring (tensor-core kernel: the tiles) during a product pass, or
+  // the threads' run sums and X by row during a product through C; the team partials of Y after it, and
+  // Y for the Gram sums (yred); the pick histogram of an AMM draw (hist, zeroed at the start of
+  // every draw)
   // (tensor-core kernel: 1024-byte aligned, as the 128-byte swizzle of its tile copies needs)
   static constexpr int region = TC ? align1024(xs + xs_bytes) : align16(xs + xs_bytes);
   static constexpr int yred = region;                                    // float [4*kThreads][K]
@@ -785,10 +785,10 @@ __device__ __noinline__ void gram_step(const float* Xs, const float* Ys, double*
 
 // Y = C·X over this team's share of C's columns (C = A·Aᵀ, ldc x ldc, zeros past m), this thread's
 // rows r0 .. r0 + 3: per column one 16-byte load of C (coalesced over the team, four columns ahead in
-// registers) against X's row (broadcast loads from `xrow`, see yq), in packed FP32 FMAs.  Bounded by the FMAs and by an
-// SM's share of the L2 (16 packed FMAs per 16 bytes).  The sums are taken in runs of 16 columns, added
-// up in this thread's slot of shared memory (`slots`, [value / 4][thread]): one FP32 chain over a
-// team's whole share made the rounding of Y the largest error of λ where the eigenvector sits on
+// registers) against X's row (broadcast loads from `xrow`, see yq), in packed FP32 FMAs.  Bounded by the
+// FMAs and by an SM's share of the L2 (16 packed FMAs per 16 bytes).  The sums are taken in runs of 16
+// columns, added up in this thread's slot of shared memory (`slots`, [value / 4][thread]): one FP32 chain
+// over a team's whole share made the rounding of Y the largest error of λ where the eigenvector sits on
 // few rows (300 x 700 with lognormal row scales: rms 1.6e-7 -> 1.2e-7).  Out of line so that its
 // registers do not compete with the other product loops'.
 template <int K>

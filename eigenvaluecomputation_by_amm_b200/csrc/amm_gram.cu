@@ -14,8 +14,8 @@
 //
 // One CTA of 512 threads per tile of 128 rows x up to 256 columns on or below the diagonal, tiles
 // taken from a queue, longest first.  256 columns because a product of 128 x N x 16 takes about as
-// long for N = 128 as for N = 256 (128 x 128 tiles: 6.7 ms for the 476 matrices of the 512-matrix
-// batch that are multiplied as C·X).  Per chunk every thread converts 2 + 4 float4 (4 consecutive
+// long for N = 128 as for N = 256 (476 matrices of the 512-matrix batch: 6.7 ms with 128 x 128 tiles, 6.3
+// with these, before the steps below).  Per chunk every thread converts 2 + 4 float4 (4 consecutive
 // rows of a column: one coalesced 16-byte load, three 8-byte stores into the 128-byte-swizzled
 // MN-major planes), one thread issues the 12 products, and while they run the threads add the chunk before from
 // tensor memory (two accumulators, two stages of planes).  The next chunk's loads are issued before
@@ -25,7 +25,8 @@
 // planes written, 144 KB read, at 128 bytes a clock).  The whole run of the 512-matrix batch: loads
 // after the barrier, 16 tensor-memory columns at a time 14.3 ms; loads before it 14.2; 8 columns at a
 // time (fewer spills) 13.2, with the loads after the barrier 13.9; 32-bit shared-memory addresses and
-// one column pointer 12.8.
+// one column pointer 12.8.  148 matrices of 512 x 2560: 0.92 ms, 810 TFLOP/s of products, the tensor
+// cores active in 43 % of the cycles, issue in 51 %, DRAM at 12 %.
 #include <cuda_runtime.h>
 
 #include <cstdint>

@@ -109,8 +109,10 @@ struct Buffers {
   double2* colsum;     // n (Σa, Σa²) of each column from the set-up pass
   double* rpart;       // nsm x 4 (x·y, y·y, y·v*, z·dx) of each CTA
   // packets of the step kernel (amm_step.cu): three floats and an epoch each
-  uint4* pk_part;      // nsm x (packets of a vector + 1): the CTAs' partial y and scalars
-  uint4* pk_y;         // packets of a vector: y; then the CTAs' shares of the Rayleigh sums
+  uint4* pk_part;      // nsm x (packets of a vector + 2): the CTAs' partial y, and their scalars
+                       // by step parity
+  uint4* pk_y;         // a block per CTA: the packets of y it owns, then its shares of the
+                       // Rayleigh sums
   uint32_t* epoch;     // epoch before the next launch's first step
   uint32_t* ticket;    // [2]: grid-barrier arrivals of the step kernel and the set-up pass;
                        // [3]: the wait probe's barrier; [0], [1]: spare

@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(kMaxThreads, 1)
             if (qq < cnt) axpy_col(qq, s_cur, coef[qq]);
         }
         if (more && ok) publish(cnt_n, (grp + 1) & 1, dn);
-        // partials of grp+1 published; every thread is done with stage grp: thread 0 refills it
+        // partials of grp+1 published; every thread is done with stage grp: the issuing warp refills it
         if (named_barrier_or(1, T, !ok)) ok = false;
         if (warp == iw && ok && grp + NS < ngroups) {
           const int c0 = (grp + NS) * GC;
