@@ -2306,17 +2306,26 @@ static double gram_run_us(const std::vector<Mat>& ms, const std::vector<GramCost
     for (size_t i = 0; i < ms.size(); ++i)
       us[i] = p * ((take[i] ? cost[i].by_c : cost[i].by_a) / cl + 17.7 +
                    0.0069 * (double)(cl - 1) * (double)ms[i].m);
-    std::sort(us.begin(), us.end(), std::greater<double>());
-    std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
     // (of 148 SMs 33 clusters of 4 and 15 of 8 are resident)
     const int clusters = std::max(1, (cl > 2 ? 9 * nsm / 10 : nsm) / cl);
-    for (int k = 0; k < clusters; ++k) free_at.push(0.0);
     double end = 0.0;
-    for (const double u : us) {
-      const double done = free_at.top() + u;
-      free_at.pop();
-      free_at.push(done);
-      end = std::max(end, done);
+    if (us.size() > 1024) {  // many: an even share, or the longest matrix
+      double sum = 0.0;
+      for (const double u : us) {
+        sum += u;
+        end = std::max(end, u);
+      }
+      end = std::max(end, sum / (double)clusters);
+    } else {
+      std::sort(us.begin(), us.end(), std::greater<double>());
+      std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+      for (int k = 0; k < clusters; ++k) free_at.push(0.0);
+      for (const double u : us) {
+        const double done = free_at.top() + u;
+        free_at.pop();
+        free_at.push(done);
+        end = std::max(end, done);
+      }
     }
     if (cl == 1 || end < best) best = end;
   }
