@@ -371,8 +371,7 @@ class BatchSolver:
               "amm_batch_vector_offsets")
         self.offsets = offs
         self.lam = torch.empty(self.count, self.nvec, dtype=torch.float64, device=self._dev)
-        # (a run leaves the vector of a matrix without a result, iters = -1, as it is)
-        self.vectors = torch.zeros(int(offs[-1]), dtype=torch.float32, device=self._dev)
+        self.vectors = torch.empty(int(offs[-1]), dtype=torch.float32, device=self._dev)
         self.iters = torch.empty(self.count, dtype=torch.int32, device=self._dev)
 
     def _descs(self, mats):
