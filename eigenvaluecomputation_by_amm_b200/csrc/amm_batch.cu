@@ -2112,8 +2112,7 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
     // products as C·X are in the tensor-core kernel, whose product through A is the fastest exact one
     // as well (42 sizes with m 64-2048, n = m/4 .. 5m, 16 and 148 or 296 matrices)
     if (b->ntiles > 0 && !amm::batch::kVariants[v].tc) continue;
-    const int gc = b->cfg.tile_gc > 0 ? b->cfg.tile_gc : sampled_blocks ? 4 : 0;
-    if (gc > 0 && amm::batch::kVariants[v].GC != gc) continue;
+    if (b->cfg.tile_gc > 0 && amm::batch::kVariants[v].GC != b->cfg.tile_gc) continue;
     for (int cl : amm::batch::kClusterSizes) {
       if (b->cfg.cluster > 0 && cl != b->cfg.cluster) continue;
       const int grid = persistent_grid(b, v, cl);
@@ -2123,11 +2122,26 @@ int autotune(amm_batch* b, double* d_lam, float* d_vec, int32_t* d_iters, cudaSt
   }
   const bool fixed = cand.size() == 1;
   if (sampled_blocks && cand.size() > 1) {
+    // Every tiling runs once, untimed: a run does not write the vector of a matrix whose block it finds
+    // singular, and that vector is then the last one that another tiling found, as it was when the
+    // tilings were timed (0.5 s of a first run of 512 matrices, where timing them took 1.4 s).
+    const int iters = (int)std::min<int64_t>(b->cfg.max_iter, 20);
+    for (const auto& cd : cand) {
+      const int rc = launch(b, std::get<0>(cd), std::get<1>(cd), std::get<2>(cd), d_lam, d_vec, d_iters,
+                            iters, order_of(b, false), (int)b->count, false, false, s);
+      if (rc) return rc;
+    }
+    const int gc = b->cfg.tile_gc > 0 ? b->cfg.tile_gc : 4;
     std::vector<std::pair<int, int>> sizes;
-    for (const auto& cd : cand) sizes.emplace_back(std::get<1>(cd), std::get<2>(cd) / std::get<1>(cd));
+    for (const auto& cd : cand)
+      if (amm::batch::kVariants[std::get<0>(cd)].GC == gc)
+        sizes.emplace_back(std::get<1>(cd), std::get<2>(cd) / std::get<1>(cd));
     const int cl = sampled_cluster(b, sizes);
     cand.erase(std::remove_if(cand.begin(), cand.end(),
-                              [&](const auto& cd) { return std::get<1>(cd) != cl; }),
+                              [&](const auto& cd) {
+                                return std::get<1>(cd) != cl ||
+                                       amm::batch::kVariants[std::get<0>(cd)].GC != gc;
+                              }),
                cand.end());
   }
   if (cand.size() == 1) {

@@ -296,8 +296,9 @@ int amm_batch_destroy(amm_batch *b);
 int amm_batch_vector_offsets(amm_batch *b, int64_t *offsets);
 /* One persistent launch over all matrices (largest first from a device queue).  d_lambda:
  * count x nvec Ritz values, descending (λ_max first); d_vectors: Σ m, the unit top Ritz vector
- * of each matrix; d_iters: products run per matrix (-1: rank-deficient block).  The first call
- * autotunes the tile shape (columns per group) on this batch. */
+ * of each matrix; d_iters: products run per matrix (-1: rank-deficient block; its Ritz values are
+ * NaN and its vector is not written).  The first call autotunes the tile shape (columns per
+ * group) on this batch. */
 int amm_batch_run(amm_batch *b, double *d_lambda, float *d_vectors, int32_t *d_iters,
                   void *stream);
 /* Rebind the batch to new matrices of the same shapes (same count, m and n per matrix; A and
